@@ -117,7 +117,9 @@ typedef struct st3d_grid_desc {
  * kernel, then one 2-D copy).  DIRECT: the scatter/gather kernels read and
  * write the host array itself over the host link; it applies to pinned host
  * arrays (cudaMallocHost, cudaHostAlloc, cudaHostRegister, st3d_host_alloc)
- * that lie inside one allocation.  AUTO takes DIRECT where it applies.
+ * that lie inside one allocation.  AUTO takes DIRECT where it applies, and
+ * moves device arrays of the context's device the same way (one pass of the
+ * scatter/gather kernel over the caller's array).
  * STRIDED: a 3-D strided copy, used when the host k halo exceeds the device
  * row pad.  STREAMED (st3d_iterate_host only): the DIRECT path with the
  * transfers and the steps overlapped in one launch -- CTAs copying planes of

@@ -355,6 +355,19 @@ int copy_field_strided(st3d_ctx* c, void* dev, void* host, bool to_device, bool 
   return ST3D_OK;
 }
 
+// The driver's range of the allocation that holds p .. p + bytes.
+bool in_one_allocation(const void* p, size_t bytes) {
+  auto attr = get_pointer_attr();
+  if (!attr) return false;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr q = (CUdeviceptr)(uintptr_t)p;
+  if (attr(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, q) != CUDA_SUCCESS ||
+      attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, q) != CUDA_SUCCESS)
+    return false;
+  return q >= start && q + bytes <= start + size;
+}
+
 // The device address of a host array the kernels may read and write
 // directly: pinned (cudaMallocHost, cudaHostAlloc, cudaHostRegister) and
 // lying inside one allocation; nullptr otherwise (pageable memory, or a range
@@ -367,16 +380,25 @@ void* direct_view(const void* host, size_t bytes) {
     return nullptr;
   }
   if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-  auto attr = get_pointer_attr();
-  if (!attr) return nullptr;
-  CUdeviceptr start = 0;
-  size_t size = 0;
-  const CUdeviceptr p = (CUdeviceptr)(uintptr_t)host;
-  if (attr(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) != CUDA_SUCCESS ||
-      attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) != CUDA_SUCCESS)
-    return nullptr;
-  if (p < start || p + bytes > start + size) return nullptr;
-  return at.devicePointer;
+  return in_one_allocation(host, bytes) ? at.devicePointer : nullptr;
+}
+
+// Whether `p` is an array in device memory that the layout kernels may read
+// or write themselves: on the context's own device, inside one allocation, on
+// an element boundary (anything else goes through the staging buffer, whose
+// copies take every address).  Staging a device array costs a pass over it
+// and, downwards, a 2-D copy that ran 2.1 TB/s: the two levels of 1024^3 FP32
+// left in 11.9 ms that way and leave in 2.9 ms directly.
+bool device_view(const st3d_ctx* c, const void* p, size_t bytes) {
+  if (c->opts.host_path != ST3D_HOST_AUTO && c->opts.host_path != ST3D_HOST_STREAMED) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == c->device &&
+         reinterpret_cast<uintptr_t>(p) % host_elem_bytes(c->opts.storage) == 0 &&
+         in_one_allocation(p, bytes);
 }
 
 // Host (reference layout) -> device field.  Staged: one contiguous copy into
@@ -394,6 +416,7 @@ int upload_field(st3d_ctx* c, void* dev, const void* host) {
   if (c->opts.host_path != ST3D_HOST_STAGED) src = direct_view(host, host_array_bytes(c));
   if (c->opts.host_path == ST3D_HOST_DIRECT && !src)
     return fail(ST3D_ERR_INVALID, "the direct host path needs a pinned host array");
+  if (!src && device_view(c, host, host_array_bytes(c))) src = host;
   if (!src) {
     int rc = ensure_stage(c);
     if (rc != ST3D_OK) return rc;
@@ -437,6 +460,7 @@ int download_field(st3d_ctx* c, const void* dev, void* host) {
   if (c->opts.host_path != ST3D_HOST_STAGED) dst = direct_view(host, host_array_bytes(c));
   if (c->opts.host_path == ST3D_HOST_DIRECT && !dst)
     return fail(ST3D_ERR_INVALID, "the direct host path needs a pinned host array");
+  if (!dst && device_view(c, host, host_array_bytes(c))) dst = host;
   if (dst) {
     c->host_path = ST3D_HOST_DIRECT;
     cudaError_t e = launch_dev_to_ref(c->eb, c->L, R, dev, dst, (int)g.zh, c->stream);

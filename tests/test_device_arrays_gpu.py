@@ -1,0 +1,51 @@
+"""Device arrays in st3d_upload and st3d_download: the layout kernels read and
+write them directly.  Bar: the values the host-array route moves, for rows
+that are and are not whole 16-byte words, FP32 and FP64, k halos beside 4, one
+thin grid, and arrays that start one element past a 16-byte boundary; points
+outside the interior rows of the target stay untouched."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import stencil3d_gb300 as S
+from stencil3d_gb300 import api
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(5, 7, 64, 4, 4, 4), (3, 9, 61, 4, 4, 4), (6, 5, 70, 4, 4, 5), (2, 3, 1, 4, 4, 16),
+         (4, 130, 257, 2, 3, 1), (1, 1, 1030, 4, 4, 2)]
+
+
+def _device(a, shift):
+    torch = pytest.importorskip("torch")
+    t = torch.empty(a.size + 4, dtype=torch.from_numpy(a).dtype, device="cuda")
+    t = t[shift:shift + a.size].view(a.shape)
+    t.copy_(torch.from_numpy(a))
+    return t
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("grid", GRIDS)
+def test_device_arrays_move_the_host_route_values(grid, shift, dtype):
+    torch = pytest.importorskip("torch")
+    np_t = np.float64 if dtype == "f64" else np.float32
+    g = S.Grid(*grid)
+    v, s, u = (O.fill_uniform(grid, 3, f, -1.0, 1.0, np_t) for f in range(3))
+    dv, ds, du = (_device(a, shift) for a in (v, s, u))
+    ov, ou = _device(np.full_like(v, -7.0), shift), _device(np.full_like(v, -7.0), shift)
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    points = 7 if min(grid[3:]) < 2 else 13
+    hv, hu = np.full_like(v, -7.0), np.full_like(u, -7.0)
+    with S.Stencil(g, points, "ref", dtype) as a, S.Stencil(g, points, "ref", dtype) as b:
+        a.upload(v, s, u)
+        assert api.lib().st3d_upload(b.handle, p(dv), p(ds), p(du)) == 0
+        for st in (a, b):
+            st.iterate(2)
+        a.download(hv, hu)
+        assert api.lib().st3d_download(b.handle, p(ov), p(ou)) == 0
+    np.testing.assert_array_equal(ov.cpu().numpy(), hv)
+    np.testing.assert_array_equal(ou.cpu().numpy(), hu)
