@@ -679,10 +679,16 @@ int plan_mma16(st3d_ctx* c, int sm_count, int max_smem) {
 // planes' scales; the halo must be zero.  which: 0 = u (time level 0),
 // 1 = v (time level -1), 2 = s.
 int upload_field16(st3d_ctx* c, int which, const void* host) {
-  int rc = ensure_stage(c);
-  if (rc != ST3D_OK) return rc;
-  if (host)
-    ST3D_CUDA(cudaMemcpyAsync(c->stage, host, host_array_bytes(c), cudaMemcpyDefault, c->stream));
+  const float* src = nullptr;
+  if (host && device_view(c, host, host_array_bytes(c))) {
+    src = static_cast<const float*>(host);
+  } else {
+    int rc = ensure_stage(c);
+    if (rc != ST3D_OK) return rc;
+    if (host)
+      ST3D_CUDA(cudaMemcpyAsync(c->stage, host, host_array_bytes(c), cudaMemcpyDefault, c->stream));
+    src = static_cast<const float*>(c->stage);
+  }
   const st3d_grid_desc& g = c->grid;
   const RefGeom R = ref_geom(g);
   const int hx = g.xh < 4 ? (int)g.xh : 4, hy = g.yh < 4 ? (int)g.yh : 4, hz = (int)g.zh;
@@ -692,10 +698,10 @@ int upload_field16(st3d_ctx* c, int which, const void* host) {
   const int buf = which == 2 ? 2 : (which == 0 ? u_index(c) : v_index(c));
   ST3D_CUDA(cudaMemsetAsync(M, 0, g.xs * sizeof(uint32_t), c->stream));
   ST3D_CUDA(cudaMemsetAsync(c->halo_max, 0, sizeof(uint32_t), c->stream));
-  cudaError_t e = launch_plane_max_ref(R, (const float*)c->stage, M, c->halo_max, hx, hy, hz, c->stream);
+  cudaError_t e = launch_plane_max_ref(R, src, M, c->halo_max, hx, hy, hz, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "plane maximum kernel");
   const int storage = (which == 2 && c->opts.storage == ST3D_F16_HILO) ? ST3D_F16 : c->opts.storage;
-  e = launch_ref_to_dev16(storage, c->L, R, (const float*)c->stage, (uint16_t*)c->fld[buf],
+  e = launch_ref_to_dev16(storage, c->L, R, src, (uint16_t*)c->fld[buf],
                           which == 2 ? nullptr : (int8_t*)c->lo[buf], M, E, hx, hy, hz, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "16-bit encode kernel");
   uint32_t halo = 0;
@@ -709,16 +715,18 @@ int upload_field16(st3d_ctx* c, int which, const void* host) {
 }
 
 int download_field16(st3d_ctx* c, int which, void* host) {
-  int rc = ensure_stage(c);
+  const bool direct = device_view(c, host, host_array_bytes(c));
+  int rc = direct ? ST3D_OK : ensure_stage(c);
   if (rc != ST3D_OK) return rc;
   const st3d_grid_desc& g = c->grid;
   const RefGeom R = ref_geom(g);
   const long long level = which == 0 ? (long long)c->lvl : (long long)c->lvl - 1;
   const int buf = which == 0 ? u_index(c) : v_index(c);
   cudaError_t e = launch_dev16_to_ref(c->opts.storage, c->L, R, (const uint16_t*)c->fld[buf],
-                                      (const int8_t*)c->lo[buf], E_level(c, level), (float*)c->stage,
-                                      (int)g.zh, c->stream);
+                                      (const int8_t*)c->lo[buf], E_level(c, level),
+                                      (float*)(direct ? host : c->stage), (int)g.zh, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "16-bit decode kernel");
+  if (direct) return ST3D_OK;
   const size_t off = ((size_t)g.xh * R.imult + (size_t)g.yh * R.jmult) * 4;
   ST3D_CUDA(cudaMemcpy2DAsync(static_cast<char*>(host) + off, R.imult * 4,
                               static_cast<const char*>(c->stage) + off, R.imult * 4,
@@ -825,16 +833,19 @@ int delta_encode_pair(st3d_ctx* c, bool u_changed) {
 }
 
 int delta_download(st3d_ctx* c, void* host, bool v) {
-  int rc = ensure_stage(c, 2);
+  const bool direct = device_view(c, host, host_array_bytes(c));
+  int rc = direct ? ST3D_OK : ensure_stage(c, 2);
   if (rc != ST3D_OK) return rc;
   c->pair_valid = false;
   const st3d_grid_desc& g = c->grid;
   const RefGeom R = ref_geom(g);
   cudaError_t e = launch_delta_to_ref(word_storage(c->opts.storage), c->L, R,
                                       (const uint16_t*)c->fld[c->ub], Eu_buf(c, c->ub),
-                                      (const uint16_t*)c->fld[3], Ed_lvl(c, c->lvl), v, stage_slot(c, 0),
-                                      (int)g.zh, c->stream, (const uint16_t*)c->lo[c->ub]);
+                                      (const uint16_t*)c->fld[3], Ed_lvl(c, c->lvl), v,
+                                      direct ? (float*)host : stage_slot(c, 0), (int)g.zh, c->stream,
+                                      (const uint16_t*)c->lo[c->ub]);
   if (e != cudaSuccess) return cuda_fail(e, "16-bit decode kernel");
+  if (direct) return ST3D_OK;
   const size_t off = ((size_t)g.xh * R.imult + (size_t)g.yh * R.jmult) * 4;
   ST3D_CUDA(cudaMemcpy2DAsync(static_cast<char*>(host) + off, R.imult * 4,
                               reinterpret_cast<const char*>(stage_slot(c, 0)) + off, R.imult * 4,
@@ -1555,10 +1566,14 @@ int st3d_upload(st3d_ctx* c, const void* v, const void* s, const void* u) {
       if (v) c->has_v = true;
     }
     if (s) {
-      c->pair_valid = false;  // s passes through slot 0
-      ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), s, host_array_bytes(c), cudaMemcpyDefault,
-                                c->stream));
-      if ((rc = encode_staged16(c, stage_slot(c, 0), nullptr, c->fld[2], M_s(c), E_s(c), "s")) !=
+      c->pair_valid = false;  // s passes through slot 0, unless it is a device array
+      const float* src = stage_slot(c, 0);
+      if (device_view(c, s, host_array_bytes(c)))
+        src = static_cast<const float*>(s);
+      else
+        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), s, host_array_bytes(c), cudaMemcpyDefault,
+                                  c->stream));
+      if ((rc = encode_staged16(c, src, nullptr, c->fld[2], M_s(c), E_s(c), "s")) !=
           ST3D_OK)
         return rc;
       c->has_s = true;

@@ -49,3 +49,39 @@ def test_device_arrays_move_the_host_route_values(grid, shift, dtype):
         assert api.lib().st3d_download(b.handle, p(ov), p(ou)) == 0
     np.testing.assert_array_equal(ov.cpu().numpy(), hv)
     np.testing.assert_array_equal(ou.cpu().numpy(), hu)
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16_hl", "f16_hilo"])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("grid", [(5, 7, 64, 4, 4, 4), (3, 70, 61, 4, 4, 4), (6, 33, 262, 4, 4, 5),
+                                  (2, 3, 1, 4, 4, 16)])
+def test_device_arrays_in_16_bit_storage(grid, shift, storage):
+    """Maxima, encoding and decoding straight from and to device arrays: the
+    host-array route's words, at rows that are and are not whole fours and
+    planes of several pieces."""
+    torch = pytest.importorskip("torch")
+    g = S.Grid(*grid)
+    fields = []
+    for f in range(3):
+        a = np.zeros(O.shape(grid), np.float32)
+        O.interior(a, grid)[...] = O.interior(O.fill_uniform(grid, 5, f, -3.0, 3.0), grid)
+        fields.append(a)
+    dev = [_device(a, shift) for a in fields]
+    out = [_device(np.full_like(fields[0], -7.0), shift) for _ in range(2)]
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    hv, hu = np.full_like(fields[0], -7.0), np.full_like(fields[0], -7.0)
+    with S.Stencil(g, 7, "wave", storage, dt=1e-3) as a, S.Stencil(g, 7, "wave", storage, dt=1e-3) as b:
+        a.upload(*fields)
+        assert api.lib().st3d_upload(b.handle, *(p(t) for t in dev)) == 0
+        for st in (a, b):
+            st.iterate(2)
+        a.download(hv, hu)
+        assert api.lib().st3d_download(b.handle, p(out[0]), p(out[1])) == 0
+        # a nonzero halo point is refused as it is on the host route
+        bad = dev[2].clone()
+        bad.view(-1)[0 if grid[3] <= 4 else -1] = 1.0
+        torch.cuda.synchronize()
+        assert api.lib().st3d_upload(b.handle, None, None, p(bad)) == S.api.ERR_UNSUPPORTED
+    np.testing.assert_array_equal(out[0].cpu().numpy(), hv)
+    np.testing.assert_array_equal(out[1].cpu().numpy(), hu)
