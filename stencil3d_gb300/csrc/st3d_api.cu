@@ -906,7 +906,7 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   *done = false;
   const int hp = c->opts.host_path;
   if (hp != ST3D_HOST_AUTO && hp != ST3D_HOST_STREAMED) return ST3D_OK;
-  if (iterations < 1 || c->opts.storage != ST3D_F32 || c->f16 || c->tb || !c->tma ||
+  if (iterations < 1 || iterations > 0x7fffffffu || c->opts.storage != ST3D_F32 || c->f16 || c->tb || !c->tma ||
       c->kernel != ST3D_KERNEL_TMA || c->tma->tj != 16 || c->tma->nv != 4 || !staged_ok(c))
     return ST3D_OK;
   const int pts = c->opts.points;
@@ -925,7 +925,8 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   const st3d_grid_desc& gd = c->grid;
   const bool wave = c->opts.mode == ST3D_MODE_WAVE;
   const int R = c->R;
-  const int T = (int)iterations;
+  // mode R takes up to kRefSteps steps each time an item is run
+  const int T = wave ? (int)iterations : (int)((iterations - 1) / kRefSteps) + 1;
   StreamPlan p;
   p.chunk = c->opts.ichunk > 0 ? c->opts.ichunk : 16;
   if (p.chunk < R) p.chunk = R;
@@ -1024,6 +1025,7 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   L.ub0 = c->ub;
   L.vb0 = c->vb;
   L.steps = T;
+  L.iterations = (int)iterations;
   L.pairs = reinterpret_cast<const int2*>(db + o_pairs);
   L.xfer = reinterpret_cast<const int4*>(db + o_xfer);
   L.nup = nup;
@@ -1050,7 +1052,7 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   // any wait's cap: the timeout plus four times the call at 100 Gpts/s and
   // the transfers at 20 GB/s, far beyond any run that makes progress
   const double pts_all = (double)gd.xs * gd.ys * gd.zs;
-  L.cap_ns = L.timeout_ns + (uint64_t)(4.0 * (pts_all * T / 100.0 + 5.0 * hbytes / 20.0));
+  L.cap_ns = L.timeout_ns + (uint64_t)(4.0 * (pts_all * iterations / 100.0 + 5.0 * hbytes / 20.0));
   L.status = c->dev_status;
   const CUtensorMap maps[5] = {c->tma->umap[0], c->tma->umap[1], c->tma->vmap[0], c->tma->vmap[1],
                                c->tma->vmap[2]};
@@ -1060,8 +1062,8 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   // upload and advances T steps; mode W swaps the pair every step
   c->has_u = c->has_v = c->has_s = true;
   c->pair_valid = false;
-  c->step = (uint64_t)T;
-  c->lvl += (uint64_t)T;
+  c->step = iterations;
+  c->lvl += iterations;
   c->launches += 1;
   if (wave && (T & 1)) {
     const int t = c->ub;
@@ -1665,7 +1667,10 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     ++c->launches;
     iterations -= T;
   }
-  for (uint32_t n = 0; n < iterations; ++n) {
+  for (uint32_t n = 0; n < iterations;) {
+    // mode R: u and s stay fixed, a launch takes many steps (2 points: v does
+    // not even depend on v, the last step is the call)
+    const uint32_t take = wave ? 1u : std::min(iterations - n, (uint32_t)kRefSteps);
     Source src;
     src.i = -1; src.j = -1; src.k = -1; src.amp = 0.0f; src.amp_d = 0.0;
     if (wave && c->opts.src_i >= 0) {
@@ -1719,16 +1724,17 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
                        c->dev_status, c->stream);
     } else if (c->kernel == ST3D_KERNEL_TMA) {
       e = launch_tma(*c->tma, c->opts.points, c->opts.mode, c->G, c->cf32, (float*)v_ptr(c),
-                     u_index(c), v_index(c), 2, src, c->dev_status, c->stream);
+                     u_index(c), v_index(c), 2, src, (int)take, c->dev_status, c->stream);
     } else {
       const void* cf = c->opts.storage == ST3D_F64 ? (const void*)&c->cf64 : (const void*)&c->cf32;
       e = launch_simple(c->opts.points, c->opts.mode, c->opts.storage, c->G, cf, v_ptr(c),
-                        u_ptr(c), c->fld[2], src, c->ichunk, c->stream);
+                        u_ptr(c), c->fld[2], src, c->ichunk, (int)take, c->stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "stencil kernel launch");
     ++c->launches;
-    ++c->step;
-    ++c->lvl;
+    n += take;
+    c->step += take;
+    c->lvl += take;
     if (wave) {
       const int t = c->ub;
       c->ub = c->vb;

@@ -147,6 +147,7 @@ struct StreamLaunch {
   const float* hin[3];  // device views of the host u, v, s
   float* hout[2];       // device views of the host u, v written back
   int ub0, vb0, steps;
+  int iterations;  // mode R: the call's steps, kRefSteps at most in each of `steps`
   const int2* pairs;
   const int4* xfer;  // uploads [0, nup), downloads [nup, nxfer)
   int nup, nxfer;
@@ -180,15 +181,19 @@ int create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cudaStream
 
 // ---- kernel launchers (st3d_kernels_*.cu) --------------------------------
 // All launch on `stream` and return the cudaGetLastError() of the launch.
+// Mode R: one launch takes up to kRefSteps steps (u and s fixed: one pass over
+// memory); `rsteps` says how many.  The limit bounds the time between two
+// arrivals on a pipeline stage, far below the bounded waits' limit.
+constexpr int kRefSteps = 1024;
 cudaError_t launch_simple(int points, int mode, int storage, const Geom& g, const void* coefs,
                           void* v, const void* u, const void* s, const Source& src,
-                          int ichunk, cudaStream_t stream);
+                          int ichunk, int rsteps, cudaStream_t stream);
 
 struct TmaPlan;
 // ubuf/vbuf/sbuf select the tensor maps of the field buffers holding u, v, s.
 cudaError_t launch_tma(const TmaPlan& plan, int points, int mode, const Geom& g, const Coefs<float>& cf,
-                       float* v, int ubuf, int vbuf, int sbuf, const Source& src, uint32_t* dev_status,
-                       cudaStream_t stream);
+                       float* v, int ubuf, int vbuf, int sbuf, const Source& src, int rsteps,
+                       uint32_t* dev_status, cudaStream_t stream);
 bool tma_config_supported(int tj, int nv);
 // Resident CTAs per SM of the TMA kernel for this configuration (0: cannot run).
 int tma_blocks_per_sm(int points, int mode, int tj, int nv, size_t smem);

@@ -47,7 +47,7 @@ constexpr int kSimpleBY = 8;   // threads along j
 template <typename T, int P, int MODE>
 __global__ void __launch_bounds__(kSimpleBX* kSimpleBY)
     k_simple(Geom g, Coefs<T> cf, T* __restrict__ v, const T* __restrict__ u,
-             const T* __restrict__ s, int src_i, int src_j, int src_k, T amp, int ichunk) {
+             const T* __restrict__ s, int src_i, int src_j, int src_k, T amp, int ichunk, int rsteps) {
   constexpr int R = (P == 25) ? 4 : (P == 13) ? 2 : 1;
   constexpr int NP = npairs_of(P);
   const int k = blockIdx.x * kSimpleBX + threadIdx.x;
@@ -90,7 +90,9 @@ __global__ void __launch_bounds__(kSimpleBX* kSimpleBY)
       T st = cf.coef0 * u0;
 #pragma unroll
       for (int p = 0; p < NP; ++p) st = fma_t<T>(cf.cf[p], pr[p], st);
-      out = fma_t<T>(s0, st, fma_t<T>(-cf.K, u0, v0));
+      // rsteps steps: u and s stay, so does st (st3d_kernels_tma.cu)
+      out = v0;
+      for (int m = 0; m < rsteps; ++m) out = fma_t<T>(s0, st, fma_t<T>(-cf.K, u0, out));
     } else {
       if (i == src_i && j == src_j && k == src_k) s0 = s0 + amp;
       const T u2 = u0 + u0;
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(256)
 
 template <typename T, int P, int MODE>
 cudaError_t launch_t(const Geom& g, const void* coefs, void* v, const void* u, const void* s,
-                     const Source& src, int ichunk, cudaStream_t stream) {
+                     const Source& src, int ichunk, int rsteps, cudaStream_t stream) {
   const Coefs<T>& cf = *static_cast<const Coefs<T>*>(coefs);
   dim3 block(kSimpleBX, kSimpleBY, 1);
   dim3 grid((g.zs + kSimpleBX - 1) / kSimpleBX, (g.ys + kSimpleBY - 1) / kSimpleBY,
@@ -202,23 +204,23 @@ cudaError_t launch_t(const Geom& g, const void* coefs, void* v, const void* u, c
   } else {
     T amp = sizeof(T) == 8 ? (T)src.amp_d : (T)src.amp;
     k_simple<T, P, MODE><<<grid, block, 0, stream>>>(g, cf, (T*)v, (const T*)u, (const T*)s,
-                                                      src.i, src.j, src.k, amp, ichunk);
+                                                      src.i, src.j, src.k, amp, ichunk, rsteps);
   }
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_typed(int points, int mode, const Geom& g, const void* coefs, void* v,
-                         const void* u, const void* s, const Source& src, int ichunk,
+                         const void* u, const void* s, const Source& src, int ichunk, int rsteps,
                          cudaStream_t stream) {
 #define ST3D_CASE(PTS)                                                                   \
   case PTS:                                                                              \
     return mode == ST3D_MODE_REF                                                         \
-               ? launch_t<T, PTS, ST3D_MODE_REF>(g, coefs, v, u, s, src, ichunk, stream) \
-               : launch_t<T, PTS, ST3D_MODE_WAVE>(g, coefs, v, u, s, src, ichunk, stream);
+               ? launch_t<T, PTS, ST3D_MODE_REF>(g, coefs, v, u, s, src, ichunk, rsteps, stream) \
+               : launch_t<T, PTS, ST3D_MODE_WAVE>(g, coefs, v, u, s, src, ichunk, rsteps, stream);
   switch (points) {
     case 2:
-      return launch_t<T, 2, ST3D_MODE_REF>(g, coefs, v, u, s, src, ichunk, stream);
+      return launch_t<T, 2, ST3D_MODE_REF>(g, coefs, v, u, s, src, ichunk, rsteps, stream);
       ST3D_CASE(7)
       ST3D_CASE(13)
       ST3D_CASE(25)
@@ -232,12 +234,12 @@ cudaError_t launch_typed(int points, int mode, const Geom& g, const void* coefs,
 
 cudaError_t launch_simple(int points, int mode, int storage, const Geom& g, const void* coefs,
                           void* v, const void* u, const void* s, const Source& src, int ichunk,
-                          cudaStream_t stream) {
+                          int rsteps, cudaStream_t stream) {
   if (ichunk <= 0) ichunk = 64;
   if (storage == ST3D_F32)
-    return launch_typed<float>(points, mode, g, coefs, v, u, s, src, ichunk, stream);
+    return launch_typed<float>(points, mode, g, coefs, v, u, s, src, ichunk, rsteps, stream);
   if (storage == ST3D_F64)
-    return launch_typed<double>(points, mode, g, coefs, v, u, s, src, ichunk, stream);
+    return launch_typed<double>(points, mode, g, coefs, v, u, s, src, ichunk, rsteps, stream);
   return cudaErrorInvalidValue;
 }
 

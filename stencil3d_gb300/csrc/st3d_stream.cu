@@ -71,6 +71,7 @@ struct StreamArgs {
   float* hout[2];       // device views of the host outputs: u, v
   int ub0, vb0;         // buffers of u and v at the call's first step
   int steps, chunk, nchunks;
+  int iterations;       // mode R: the call's steps, up to kRefSteps in each of `steps`
   int ntk, ntiles;      // tiles per plane along k, tiles per plane
   const int2* pairs;    // (step, chunk) in wavefront order
   int npairs;
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__((kSTJ + 1) * 32, 1)
     const int vb = (MODE == ST3D_MODE_WAVE) ? (ub ^ 1) : a.vb0;
     float* vrow = a.fld[vb] + g.org + (long long)j * g.sj + k;
     const float amp = a.amps ? a.amps[t] : 0.0f;
+    const int rsteps = min(kRefSteps, a.iterations - t * kRefSteps);  // mode R
     bool ok = true;
     for (int n0 = 0; n0 < nsteps && ok; n0 += QN) {
 #pragma unroll
@@ -527,8 +529,11 @@ __global__ void __launch_bounds__((kSTJ + 1) * 32, 1)
           P4 ss = {make_float2(s4.x, s4.y), make_float2(s4.z, s4.w)};
           P4 xo;
           if (MODE == ST3D_MODE_REF) {
-            const P4 tq = fma4(splat(-a.cf.K), cu, vv);
-            xo = {__ffma2_rn(ss.a, acc.a, tq.a), __ffma2_rn(ss.b, acc.b, tq.b)};
+            xo = vv;
+            for (int m = 0; m < rsteps; ++m) {
+              const P4 tq = fma4(splat(-a.cf.K), cu, xo);
+              xo = {__ffma2_rn(ss.a, acc.a, tq.a), __ffma2_rn(ss.b, acc.b, tq.b)};
+            }
           } else {
             if (i == a.src_i && j == a.src_j && (unsigned)(a.src_k - k) < 4u) {
               const int cc = a.src_k - k;
@@ -643,6 +648,7 @@ cudaError_t launch_stream(int points, int mode, const StreamPlan& p, const CUten
   a.ub0 = L.ub0;
   a.vb0 = L.vb0;
   a.steps = L.steps;
+  a.iterations = L.iterations;
   a.chunk = p.chunk;
   a.nchunks = p.nchunks;
   a.ntk = p.ntk;
