@@ -64,6 +64,10 @@ def candidates(points, mode, storage, zero_halo=False):
         for ic in (0, 64, 256):
             out.append({"kernel": "tma", "tile_j": tj, "stages": nv, "ichunk": ic})
     out.append({"kernel": "simple", "ichunk": 64})
+    if mode == "wave":
+        # the library's own choice, which may take several steps a launch (no
+        # shape of the one-step kernel named)
+        out.append({"kernel": "tma"})
     if zero_halo and mode == "wave":
         # the fused depths the library serves: (T - 1) * R <= 8
         for T in ((2, 4) if points in (7, 13) else (2,)):

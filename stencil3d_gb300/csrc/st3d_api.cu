@@ -898,6 +898,121 @@ int plan_tb(st3d_ctx* c, int sm_count) {
   return ST3D_OK;
 }
 
+// Several wave steps a launch: FP32 wave contexts on the TMA kernel whose
+// options ask for no tile height, unit length or pipeline depth (those name
+// the one-step kernel's shape).  Without the memory or the maps for it the
+// context steps one launch at a time.
+void setup_wave(st3d_ctx* c, int sm_count) {
+  const st3d_opts& o = c->opts;
+  if (o.mode != ST3D_MODE_WAVE || o.storage != ST3D_F32 || !c->tma || c->tma->tj != 16 || c->tb ||
+      o.ichunk > 0 || o.stages > 0 || o.tile_j > 0)
+    return;
+  int coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+  if (!coop) return;
+  WavePlan* w = new (std::nothrow) WavePlan();
+  if (!w) return;
+  w->ctas = sm_count * std::min(wave_blocks_per_sm(o.points, false), wave_blocks_per_sm(o.points, true));
+  int ok = w->ctas < 2 ? ST3D_ERR_UNSUPPORTED : ST3D_OK;
+  long long most = 0;
+  for (int n = 0; n < 2 && ok == ST3D_OK; ++n) {
+    WaveShape& sh = w->shape[n];
+    const int tj = wave_tile_rows(n), tk = wave_tile_cols(n);
+    const long long ntk = ((long long)c->L.zs + tk - 1) / tk, Q = ((long long)c->L.ys + tj - 1) / tj * ntk;
+    if (Q > (1 << 18)) ok = ST3D_ERR_UNSUPPORTED;
+    sh.ntk = (int)ntk;
+    sh.Q = (int)Q;
+    most = std::max(most, Q);
+    for (int f = 0; f < 3 && ok == ST3D_OK; ++f) {
+      if (f < 2)
+        ok = encode_map(&sh.umap[f], c->fld[f], c->L, tk + 2 * kTmaKHalo, tj + 2 * c->R, kTmaKHalo, c->L.pj);
+      if (ok == ST3D_OK) ok = encode_map(&sh.vmap[f], c->fld[f], c->L, tk, tj, 0, 0);
+    }
+  }
+  if (ok == ST3D_OK) {
+    // a progress word per step and column: 8 MB at most, but 8 steps
+    w->max_steps = (int)std::min<long long>(kWaveSteps, std::max(8LL, (1LL << 16) / most));
+    w->words_n = wave_words(w->max_steps, (int)most);
+    if (cudaMalloc(&w->words, w->words_n * sizeof(int)) != cudaSuccess) ok = ST3D_ERR_NOMEM;
+  }
+  if (ok != ST3D_OK) {
+    cudaGetLastError();
+    delete w;
+    return;
+  }
+  c->wave = w;  // its words, like the other scratch, are not counted in c->bytes
+}
+
+// The shape of a launch of `steps` wave steps; false: one step a launch is
+// the better choice.  The times compared, in microseconds, are fitted to
+// measurements on a GB300 (FP32, 20 to 40 steps, device time):
+//   several steps: a CTA takes a plane of its column in 0.34 / 0.38 / 0.60 us
+//     (7 / 13 / 25 points) while the three fields fit L2, 0.47 / 0.48 / 0.62
+//     up to 300 MB and 0.55 / 0.56 / 0.62 beyond, where 4 and 5 levels are
+//     best (7 points 512^3, Gpts/s with 2 / 3 / 4 / 5 / 6 levels: 496 / 521 /
+//     549 / 567 / 506; 25 points, 1024^2 planes: 449 / 436 / 458 / 447 / 375);
+//     several turns below 300 MB 15 % more (13 points 301 x 187 x 423: 48
+//     columns at once in 3 levels 1044 us, 38 at a time in 4 levels 1160),
+//     30 % with more than 5 levels; a column whose next level waits for the
+//     next turn finds its planes gone from L2 (shift of S columns: 25 points
+//     343 x 341 x 1412, 23 of 76: 2937 us against 2539 for single steps);
+//     a level starts 6.5 us after the one before; 32 x 64 tiles take 5 % more
+//     a plane (25 points, 1024^2 planes 431 against 458 Gpts/s) and pay off
+//     where they pad less (528^3: 417 against 399);
+//   one step a launch: its units' planes (with R warm-up planes) at 0.76 us
+//     where the tiles are full (padding costs no HBM bytes), 0.5 in L2, and
+//     3.5 us a launch.
+// Measured (one step a launch -> several): 7 points 256^3 x 20 937 -> 590 us,
+// 13 points 301 x 187 x 423 x 20 1413 -> 1044, 25 points 528^3 x 40 15930 ->
+// 14113; 7 points 128^3 x 20 stays at one (145 against 159).
+bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w) {
+  if (!c->wave || steps < 2) return false;
+  const int n = (int)steps, R = c->R, xs = (int)c->L.xs;
+  const double bytes = 12.0 * c->grid.xs * c->grid.ys * c->grid.zs;
+  const int size = bytes < 1.0e8 ? 0 : bytes < 3.0e8 ? 1 : 2;
+  static const double plane_us[3][3] = {{0.34, 0.47, 0.55}, {0.38, 0.48, 0.56}, {0.60, 0.62, 0.62}};
+  const double tau = plane_us[R == 1 ? 0 : R == 2 ? 1 : 2][size];
+  static const double levels[7] = {0.0, 0.0, 1.08, 1.05, 1.0, 1.0, 1.18};
+  double best = 1e300;
+  int best_T = 0, best_n = 0;
+  for (int nar = 0; nar < 2; ++nar) {
+    const int Q = c->wave->shape[nar].Q, ntk = c->wave->shape[nar].ntk;
+    for (int T = 2; T <= std::min({n, c->wave->ctas, 24}); ++T) {
+      const int S = std::min(Q, c->wave->ctas / T);
+      const long long shift = Q <= S ? 0 : ntk;
+      // every dependency at the same or an earlier place of the sequence
+      if (shift && Q < ntk + (T - 1) * shift) break;
+      const long long passes = (n + T - 1) / T, turns = (passes * Q + (T - 1) * shift + S - 1) / S;
+      const double us = turns * (xs + 2.0 * R) * tau * (nar ? 1.05 : 1.0) *
+                            (size == 2 ? levels[std::min(T, 6)] : !shift ? 1.0 : T > 5 ? 1.3 : 1.15) *
+                            (1.0 + 0.4 * std::max(0.0, (double)shift / S - 0.2)) +
+                        6.5 * (T - 1) + 12.0;
+      if (us < best) {
+        best = us;
+        best_T = T;
+        best_n = nar;
+      }
+    }
+  }
+  const TmaPlan& p = *c->tma;
+  const double fill = (double)c->L.ys * c->L.zs / ((double)p.ntj * p.tj * p.ntk * kTmaTK);
+  const double one = 3.5 + (double)((p.units + p.grid - 1) / p.grid) * (p.ichunk + R) *
+                               (size ? 0.76 * (0.2 + 0.8 * fill) : 0.5);
+  if (!best_T || best > 0.93 * n * one) return false;
+  *w = *c->wave;
+  w->narrow = best_n;
+  w->T = best_T;
+  const int Q = w->shape[best_n].Q;
+  w->S = std::min(Q, w->ctas / best_T);
+  w->shift = Q <= w->S ? 0 : w->shape[best_n].ntk;
+  // beyond R + 1 planes, or the slowest of two neighbours could wait for the
+  // other; unbounded (7 points 256^3, 201 MB: 590 against 618 us) where L2
+  // has room (13 points 301 x 187 x 423, 286 MB: 1149 against 1044)
+  w->couple = bytes > 2.4e8 ? 18 + 2 * R : 1 << 28;
+  w->limit_ns = 4000000000ull + (uint64_t)(bytes / 12.0 * n / 2.5);
+  return true;
+}
+
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and
 // download in one cooperative launch.  *done = false (and nothing enqueued)
 // where it does not apply; the caller then runs the phases one by one.
@@ -1440,6 +1555,7 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
                             "the TMA kernel cannot run with this configuration"));
     }
   }
+  setup_wave(c, sm);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return cleanup(fail(ST3D_ERR_CUDA, "initial synchronize failed"));
   *out = c;
@@ -1460,6 +1576,8 @@ int st3d_destroy(st3d_ctx* c) {
   if (c->dev_status) cudaFree(c->dev_status);
   if (c->stage) cudaFree(c->stage);
   if (c->stream_buf) cudaFree(c->stream_buf);
+  if (c->wave) cudaFree(c->wave->words);
+  delete c->wave;
   for (int f = 0; f < 2; ++f)
     if (c->lo[f]) cudaFree(c->lo[f]);
   if (c->E) cudaFree(c->E);
@@ -1668,6 +1786,35 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     iterations -= T;
   }
   for (uint32_t n = 0; n < iterations;) {
+    WavePlan wp;
+    const uint32_t many = c->wave ? std::min(iterations - n, (uint32_t)c->wave->max_steps) : 0u;
+    if (plan_wave(c, many, &wp)) {
+      Source src;
+      src.i = c->opts.src_i; src.j = c->opts.src_j; src.k = c->opts.src_k;
+      src.amp = 0.0f; src.amp_d = 0.0;
+      float amps[kWaveSteps];
+      for (uint32_t m = 0; m < many; ++m)
+        amps[m] = src.i >= 0 ? (float)st3d_ricker((double)(c->step + m) * c->opts.dt, c->opts.src_f,
+                                                  c->opts.src_t0)
+                             : 0.0f;
+      float* const fld[2] = {(float*)c->fld[0], (float*)c->fld[1]};
+      cudaError_t e = launch_wave(wp, c->opts.points, c->G, c->cf32, fld, c->ub, (int)many, src, amps,
+                                  c->dev_status, c->stream);
+      if (e == cudaErrorCooperativeLaunchTooLarge) {
+        // fewer SMs than the device reports (a partitioned GPU): one step a
+        // launch from here on
+        cudaGetLastError();
+        c->wave->ctas = 0;
+        continue;
+      }
+      if (e != cudaSuccess) return cuda_fail(e, "wave pipeline launch");
+      if (many & 1) std::swap(c->ub, c->vb);
+      ++c->launches;
+      n += many;
+      c->step += many;
+      c->lvl += many;
+      continue;
+    }
     // mode R: u and s stay fixed, a launch takes many steps (2 points: v does
     // not even depend on v, the last step is the call)
     const uint32_t take = wave ? 1u : std::min(iterations - n, (uint32_t)kRefSteps);

@@ -14,6 +14,7 @@ struct st3d_ctx {
   using TmaPlan = st3d::TmaPlan;
   using Tma16Plan = st3d::Tma16Plan;
   using TbPlan = st3d::TbPlan;
+  using WavePlan = st3d::WavePlan;
   template <typename C>
   using Coefs = st3d::Coefs<C>;
 
@@ -71,6 +72,8 @@ struct st3d_ctx {
   Coefs<float> cf32;
   Coefs<double> cf64;
   size_t bytes = 0;
+  // several wave steps a launch (st3d_kernels_wave.cu); nullptr: one a launch
+  WavePlan* wave = nullptr;
   // the streamed drop-in call (st3d_stream.cu): its queues, counters and
   // amplitudes on the device, and their host copies (kept until the next call)
   void* stream_buf = nullptr;

@@ -198,6 +198,18 @@ bool tma_config_supported(int tj, int nv);
 // Resident CTAs per SM of the TMA kernel for this configuration (0: cannot run).
 int tma_blocks_per_sm(int points, int mode, int tj, int nv, size_t smem);
 
+// Many FP32 wave steps in one launch (st3d_kernels_wave.cu).
+constexpr int kWaveSteps = 256;  // steps of one launch at most (the amplitudes are kernel arguments)
+struct WavePlan;
+int wave_tile_rows(bool narrow);
+int wave_tile_cols(bool narrow);
+int wave_blocks_per_sm(int points, bool narrow);
+// Words of device memory a launch of that many steps keeps its progress in.
+size_t wave_words(int steps, int columns);
+cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
+                        float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
+                        uint32_t* dev_status, cudaStream_t stream);
+
 // Reference layout (staging buffer) <-> library layout, element size eb.
 cudaError_t launch_ref_to_dev(int eb, const Layout& L, const RefGeom& R, const void* stage,
                               void* dst, int hx, int hy, int hz, cudaStream_t stream);

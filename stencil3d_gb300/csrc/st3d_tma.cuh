@@ -102,6 +102,27 @@ struct TbPlan {
   CUtensorMap vmap[5];
 };
 
+// Plan of the multi-step wave kernel (st3d_kernels_wave.cu).  The two tile
+// shapes with their maps and columns, and the progress words, belong to the
+// context; shape, T, S, shift and couple are set for each launch.
+struct WaveShape {
+  int ntk = 0, Q = 0;        // tiles along k, columns
+  CUtensorMap umap[2];       // halo box over the u/v pair
+  CUtensorMap vmap[3];       // interior box over the pair and s
+};
+struct WavePlan {
+  WaveShape shape[2];        // 16 x 128 and 32 x 64 tiles
+  int ctas = 0;              // CTAs the GPU holds at once
+  int max_steps = 0;         // steps the words are enough for
+  int narrow = 0;            // the shape taken
+  int T = 1, S = 1;          // levels, columns at work in each
+  int shift = 0;             // columns a level starts behind the one before
+  int couple = 0;            // planes a column of level 0 may be ahead of its neighbours
+  int* words = nullptr;      // progress words (device)
+  size_t words_n = 0;
+  uint64_t limit_ns = 4000000000ull;
+};
+
 // Planes per work unit: the chunk length that minimises the modelled time
 // ceil(units / ctas) * (ichunk + R/2) (a unit's 2R warm-up steps load only u,
 // about a quarter of a full step's bytes), i.e. balance across the persistent
