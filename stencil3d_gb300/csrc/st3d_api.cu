@@ -1875,7 +1875,7 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     } else {
       const void* cf = c->opts.storage == ST3D_F64 ? (const void*)&c->cf64 : (const void*)&c->cf32;
       e = launch_simple(c->opts.points, c->opts.mode, c->opts.storage, c->G, cf, v_ptr(c),
-                        u_ptr(c), c->fld[2], src, c->ichunk, (int)take, c->stream);
+                        u_ptr(c), c->fld[2], src, c->opts.ichunk, (int)take, c->stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "stencil kernel launch");
     ++c->launches;

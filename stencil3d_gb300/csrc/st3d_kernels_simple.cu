@@ -28,6 +28,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "st3d_f64.cuh"
 #include "st3d_internal.h"
 
 namespace st3d {
@@ -65,6 +66,34 @@ __global__ void __launch_bounds__(kSimpleBX* kSimpleBY)
     const long long x = col + (long long)i * g.si;
     const T* c = u + x;
     const T u0 = q[R];
+    if constexpr (sizeof(T) == 8 && MODE == ST3D_MODE_WAVE) {
+      // FP64 is the bound: the two sums of a pair run as integer arithmetic
+      // where the operands' exponents allow it (st3d_f64.cuh), the
+      // multiply-adds on the FP64 unit
+      const Twice tw = twice_of(u0);
+      const T v0 = v[x];
+      T s0 = __ldg(s + x);
+      T lap = T(0);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int ax = pair_axis(P, p);
+        const int r = pair_r(P, p);
+        const T a = ax == 0 ? q[R - r] : __ldg(c - (long long)r * (ax == 1 ? g.sj : 1));
+        const T b = ax == 0 ? q[R + r] : __ldg(c + (long long)r * (ax == 1 ? g.sj : 1));
+        const Bits64 ba = bits_of(a), bb = bits_of(b);
+        int E;
+        T d;
+        if (!pair_fits(ba, bb, tw, &E) || !pair_diff_bits(ba, bb, tw, E, &d)) d = (a + b) - (u0 + u0);
+        lap = p == 0 ? cf.cf[0] * d : fma_t<T>(cf.cf[p], d, lap);
+      }
+      if (i == src_i && j == src_j && k == src_k) s0 = s0 + amp;
+      T t = fma_t<T>(T(2), u0, -v0);  // 2u - v, rounded once as the difference is
+      t = fma_t<T>(cf.c1, lap, t);
+      v[x] = fma_t<T>(cf.c2, s0, t);
+#pragma unroll
+      for (int m = 0; m < 2 * R; ++m) q[m] = q[m + 1];
+      continue;
+    }
     T pr[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
@@ -183,11 +212,50 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Planes per block where the caller names none (ichunk 0): the chunk whose
+// blocks fill the GPU's last round best, each with its 2R planes of queue to
+// load first (about a tenth of a plane's time each).  FP64, 25 points, 256^3:
+// 64 planes make 1.7 rounds of blocks, 853 us a step; 37 planes 2.9 rounds,
+// 792 us.  7 points 64^3, where 64 planes were 16 blocks: 72 -> 13 us.
+int pick_chunk(long long columns, int xs, int slots, int R) {
+  int best = 64;
+  double cost = 1e300;
+  for (int nz = 1; nz <= xs; ++nz) {
+    const int chunk = (xs + nz - 1) / nz;
+    if (chunk > 256) continue;
+    if (chunk < 8 && nz > 1) break;
+    const long long rounds = (columns * ((xs + chunk - 1) / chunk) + slots - 1) / slots;
+    const double c = (double)rounds * (chunk + 0.2 * R);
+    if (c < 0.999 * cost) {
+      cost = c;
+      best = chunk;
+    }
+  }
+  return best;
+}
+
 template <typename T, int P, int MODE>
 cudaError_t launch_t(const Geom& g, const void* coefs, void* v, const void* u, const void* s,
                      const Source& src, int ichunk, int rsteps, cudaStream_t stream) {
   const Coefs<T>& cf = *static_cast<const Coefs<T>*>(coefs);
   dim3 block(kSimpleBX, kSimpleBY, 1);
+  if (ichunk <= 0) {
+    ichunk = 64;
+    if constexpr (P != 2) {
+      static const int per_sm = [] {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_simple<T, P, MODE>, kSimpleBX * kSimpleBY, 0) !=
+            cudaSuccess)
+          cudaGetLastError();
+        return n;
+      }();
+      int dev = 0, sm = 0;
+      if (cudaGetDevice(&dev) == cudaSuccess &&
+          cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sm * per_sm > 0)
+        ichunk = pick_chunk((long long)((g.zs + kSimpleBX - 1) / kSimpleBX) * ((g.ys + kSimpleBY - 1) / kSimpleBY),
+                            g.xs, sm * per_sm, P == 25 ? 4 : P == 13 ? 2 : 1);
+    }
+  }
   dim3 grid((g.zs + kSimpleBX - 1) / kSimpleBX, (g.ys + kSimpleBY - 1) / kSimpleBY,
             (g.xs + ichunk - 1) / ichunk);
   if constexpr (P == 2) {
@@ -235,7 +303,6 @@ cudaError_t launch_typed(int points, int mode, const Geom& g, const void* coefs,
 cudaError_t launch_simple(int points, int mode, int storage, const Geom& g, const void* coefs,
                           void* v, const void* u, const void* s, const Source& src, int ichunk,
                           int rsteps, cudaStream_t stream) {
-  if (ichunk <= 0) ichunk = 64;
   if (storage == ST3D_F32)
     return launch_typed<float>(points, mode, g, coefs, v, u, s, src, ichunk, rsteps, stream);
   if (storage == ST3D_F64)
