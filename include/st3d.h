@@ -342,7 +342,9 @@ double st3d_ricker(double t, double f, double t0);
  *                          (grid, tile, chunk) items from a device work queue;
  *   ST3D_BATCH_GRAPH       the persistent schedule with the whole time loop
  *                          captured once in a CUDA graph (cached by step
- *                          count) and replayed;
+ *                          count) and replayed; grids whose steps run faster
+ *                          as multi-step launches of their own (no unit
+ *                          length given) get those in the same graph;
  *   ST3D_BATCH_PIPELINED   every step of the call in ONE persistent launch:
  *                          a per-(step, grid) counter of finished work items
  *                          lets a grid start its next step as soon as its own

@@ -898,15 +898,15 @@ int plan_tb(st3d_ctx* c, int sm_count) {
   return ST3D_OK;
 }
 
-// Several wave steps a launch: FP32 wave contexts on the TMA kernel whose
-// options ask for no tile height, unit length or pipeline depth (those name
-// the one-step kernel's shape).  Without the memory or the maps for it the
-// context steps one launch at a time.
+}  // namespace
+
+namespace st3d {
+
+// Several wave steps a launch: FP32 wave contexts on the TMA kernel.  Without
+// the memory or the maps for it the context steps one launch at a time.
 void setup_wave(st3d_ctx* c, int sm_count) {
   const st3d_opts& o = c->opts;
-  if (o.mode != ST3D_MODE_WAVE || o.storage != ST3D_F32 || !c->tma || c->tma->tj != 16 || c->tb ||
-      o.ichunk > 0 || o.stages > 0 || o.tile_j > 0)
-    return;
+  if (c->wave || o.mode != ST3D_MODE_WAVE || o.storage != ST3D_F32 || !c->tma || c->tb) return;
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
   if (!coop) return;
@@ -965,7 +965,7 @@ void setup_wave(st3d_ctx* c, int sm_count) {
 // Measured (one step a launch -> several): 7 points 256^3 x 20 937 -> 590 us,
 // 13 points 301 x 187 x 423 x 20 1413 -> 1044, 25 points 528^3 x 40 15930 ->
 // 14113; 7 points 128^3 x 20 stays at one (145 against 159).
-bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w) {
+bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, bool any) {
   if (!c->wave || steps < 2) return false;
   const int n = (int)steps, R = c->R, xs = (int)c->L.xs;
   const double bytes = 12.0 * c->grid.xs * c->grid.ys * c->grid.zs;
@@ -998,7 +998,8 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w) {
   const double fill = (double)c->L.ys * c->L.zs / ((double)p.ntj * p.tj * p.ntk * kTmaTK);
   const double one = 3.5 + (double)((p.units + p.grid - 1) / p.grid) * (p.ichunk + R) *
                                (size ? 0.76 * (0.2 + 0.8 * fill) : 0.5);
-  if (!best_T || best > 0.93 * n * one) return false;
+  if (!best_T || (!any && best > 0.93 * n * one)) return false;
+  if (est_us) *est_us = best;
   *w = *c->wave;
   w->narrow = best_n;
   w->T = best_T;
@@ -1012,6 +1013,10 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w) {
   w->limit_ns = 4000000000ull + (uint64_t)(bytes / 12.0 * n / 2.5);
   return true;
 }
+
+}  // namespace st3d
+
+namespace {
 
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and
 // download in one cooperative launch.  *done = false (and nothing enqueued)
@@ -1555,7 +1560,9 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
                             "the TMA kernel cannot run with this configuration"));
     }
   }
-  setup_wave(c, sm);
+  // (options that name a tile height, unit length or pipeline depth ask for
+  // the one-step kernel in that shape)
+  if (c->opts.tile_j <= 0 && c->opts.ichunk <= 0 && c->opts.stages <= 0) setup_wave(c, sm);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return cleanup(fail(ST3D_ERR_CUDA, "initial synchronize failed"));
   *out = c;

@@ -16,6 +16,13 @@
 // graph and replayed.  The baseline schedule launches the single-grid kernel
 // once per grid per step.
 //
+// The graph schedule may split the batch: a grid whose steps run faster as
+// multi-step launches of its own (st3d_kernels_wave.cu, planes reused in L2)
+// gets those, one grid after the other, and the rest step together as above;
+// everything is captured in the one graph.  24 grids of 64..320 points a side,
+// 50 steps: 28.3 ms as one queue (HBM-bound at 327 Gpts/s), 23.3 ms split; 64
+// such grids 361 -> 392 Gpts/s; batches of small grids stay in the queue.
+//
 // The pipelined schedule runs every step of a call in ONE persistent launch:
 // the queue runs over (step, item) in step-major order, and a per-(step,
 // grid) counter of finished items orders the steps of each grid.  Before a
@@ -428,12 +435,17 @@ struct st3d_batch {
   cudaEvent_t amps_copied = nullptr;  // the last copy out of h_amps has been done
   uint32_t* d_status = nullptr;
   std::vector<BatchGrid> grids;
+  std::vector<int2> items;  // the queue of one step, largest grid first
   int total_items = 0;
-  int ctas = 0;
+  int ctas = 0, max_ctas = 1;  // per launch; what the GPU holds
   size_t smem = 0;
   uint64_t launches = 0;
   uint64_t points = 0;
-  std::map<uint32_t, cudaGraphExec_t> graphs;  // by step count
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    int2* items = nullptr;  // the queue of the grids that step together (device)
+  };
+  std::map<uint32_t, Graph> graphs;  // by step count
   int device = -1;  // CUDA device ordinal of every grid (opts.device), -1: current
 };
 
@@ -450,7 +462,11 @@ int bfail(int status, const char* msg) { return set_error(status, "%s", msg); }
   } while (0)
 
 void destroy_graphs(st3d_batch* b) {
-  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
+  if (!b->graphs.empty()) cudaStreamSynchronize(b->stream);
+  for (auto& kv : b->graphs) {
+    cudaGraphExecDestroy(kv.second.exec);
+    if (kv.second.items) cudaFree(kv.second.items);
+  }
   b->graphs.clear();
 }
 
@@ -506,14 +522,14 @@ int stage_call(st3d_batch* b, uint32_t steps) {
   return ST3D_OK;
 }
 
-int enqueue_persistent(st3d_batch* b, uint32_t steps) {
+int enqueue_persistent(st3d_batch* b, uint32_t steps, const int2* items, int total_items) {
   B_CUDA(cudaMemsetAsync(b->d_head, 0, (size_t)steps * sizeof(int), b->stream));
   for (uint32_t t = 0; t < steps; ++t) {
     BatchArgs a;
     a.grids = b->d_grids;
     a.maps = b->d_maps;
-    a.items = b->d_items;
-    a.total_items = b->total_items;
+    a.items = items;
+    a.total_items = total_items;
     a.n_grids = (int)b->ctx.size();
     a.head = b->d_head + t;
     a.amps = b->d_amps;
@@ -522,10 +538,122 @@ int enqueue_persistent(st3d_batch* b, uint32_t steps) {
     a.done = nullptr;
     a.timeout_ns = 4000000000ull;
     a.status = b->d_status;
-    k_batch<<<b->ctas, (kBTJ + 1) * 32, b->smem, b->stream>>>(a);
+    k_batch<<<std::min(b->ctas, total_items), (kBTJ + 1) * 32, b->smem, b->stream>>>(a);
     B_CUDA(cudaGetLastError());
   }
   return ST3D_OK;
+}
+
+// Which grids leave the shared queue of the graph schedule for multi-step
+// launches of their own: the split with the least estimated time.  A step of
+// the queue takes its units' planes (with their warm-up) at 0.6 us over the
+// CTAs, 3 us for the launch and a quarter of the longest unit for the tail
+// (24 grids 567 us a step, their 7 slowest alone 238).  Grids are taken in the
+// order of what their own launches save.
+std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
+  const size_t n = b->ctx.size();
+  std::vector<double> own(n, 1e300), share(n), unit(n);
+  std::vector<int> order;
+  for (size_t gi = 0; gi < n; ++gi) {
+    const st3d_ctx* c = b->ctx[gi];
+    const st3d_grid_desc& g = c->grid;
+    const BatchGrid& G = b->grids[gi];
+    const double chunks = (double)G.units / G.ntjk;
+    share[gi] = 0.6 * G.ntjk * (g.xs + chunks * 2 * c->R) / b->max_ctas;
+    unit[gi] = 0.6 * (std::min<int>((int)g.xs, G.ichunk) + 2 * c->R);
+    if (!c->wave) continue;
+    double us = 0.0;
+    WavePlan w;
+    for (uint32_t done = 0; done < steps;) {
+      const uint32_t many = std::min(steps - done, (uint32_t)c->wave->max_steps);
+      double part = 0.0;
+      if (!plan_wave(c, many, &w, &part, true)) {
+        us = 1e300;
+        break;
+      }
+      us += part;
+      done += many;
+    }
+    own[gi] = us;
+    if (us < 1e299) order.push_back((int)gi);
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return own[x] / share[x] < own[y] / share[y];
+  });
+  std::vector<char> alone(n, 0), best(n, 0);
+  double best_us = 1e300, mine = 0.0;
+  for (size_t k = 0; k <= order.size(); ++k) {
+    if (k > 0) {
+      alone[order[k - 1]] = 1;
+      mine += own[order[k - 1]];
+    }
+    double sum = 0.0, longest = 0.0;
+    for (size_t gi = 0; gi < n; ++gi)
+      if (!alone[gi]) {
+        sum += share[gi];
+        longest = std::max(longest, unit[gi]);
+      }
+    const double us = mine + (sum > 0.0 ? steps * (std::max(sum + 0.25 * longest, 0.75 * longest) + 3.0) : 0.0);
+    if (us < best_us) {
+      best_us = us;
+      best = alone;
+    }
+  }
+  return best;
+}
+
+// The multi-step launches of the grids that run alone, u's buffer and the
+// amplitudes read from device memory (the launches are captured).
+int enqueue_alone(st3d_batch* b, uint32_t steps, const std::vector<char>& alone) {
+  const int n = (int)b->ctx.size();
+  for (int gi = 0; gi < n; ++gi) {
+    if (!alone[gi]) continue;
+    st3d_ctx* c = b->ctx[gi];
+    Source src;
+    src.i = c->opts.src_i; src.j = c->opts.src_j; src.k = c->opts.src_k;
+    src.amp = 0.0f; src.amp_d = 0.0;
+    float* const fld[2] = {(float*)c->fld[0], (float*)c->fld[1]};
+    for (uint32_t done = 0; done < steps;) {
+      const uint32_t many = std::min(steps - done, (uint32_t)c->wave->max_steps);
+      WavePlan w;
+      if (!plan_wave(c, many, &w, nullptr, true)) return bfail(ST3D_ERR_CUDA, "no multi-step launch");
+      B_CUDA(launch_wave_dev(w, c->opts.points, c->G, c->cf32, fld, &b->d_grids[gi].cur0, (int)(done & 1),
+                             (int)many, src, b->d_amps + (size_t)done * n + gi, n, c->dev_status, b->stream));
+      done += many;
+    }
+  }
+  return ST3D_OK;
+}
+
+// Captures one call of `steps` steps.
+int capture_graph(st3d_batch* b, uint32_t steps, const std::vector<char>& alone, st3d_batch::Graph* out) {
+  std::vector<int2> items;
+  for (const int2& it : b->items)
+    if (!alone[it.x]) items.push_back(it);
+  if (!items.empty()) {
+    B_CUDA(cudaMalloc(&out->items, items.size() * sizeof(int2)));
+    B_CUDA(cudaMemcpyAsync(out->items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice,
+                           b->stream));
+    B_CUDA(cudaStreamSynchronize(b->stream));
+  }
+  cudaGraph_t graph = nullptr;
+  B_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = enqueue_alone(b, steps, alone);
+  if (rc == ST3D_OK && !items.empty()) rc = enqueue_persistent(b, steps, out->items, (int)items.size());
+  cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+  if (rc == ST3D_OK && e != cudaSuccess)
+    rc = set_error(ST3D_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
+  if (rc == ST3D_OK) {
+    e = cudaGraphInstantiate(&out->exec, graph, 0);
+    if (e != cudaSuccess) rc = set_error(ST3D_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
+  }
+  if (graph) cudaGraphDestroy(graph);
+  if (rc != ST3D_OK) {
+    cudaGetLastError();
+    if (out->items) cudaFree(out->items);
+    out->items = nullptr;
+  }
+  return rc;
 }
 
 // All steps of the call in one persistent launch: one queue over (step,
@@ -626,6 +754,7 @@ int st3d_batch_create(uint32_t n, const st3d_grid_desc* grids, const st3d_opts* 
     rc = create_context(&grids[gi], &o, b->stream, &c);
     if (rc != ST3D_OK) return cleanup(rc);
     b->ctx.push_back(c);
+    if (o.ichunk <= 0) setup_wave(c, sm);  // a unit length given asks for the queue
     BatchGrid& G = b->grids[gi];
     memset(&G, 0, sizeof G);
     G.g = c->G;
@@ -668,7 +797,7 @@ int st3d_batch_create(uint32_t n, const st3d_grid_desc* grids, const st3d_opts* 
     const double wy = (double)b->ctx[y]->grid.xs * b->ctx[y]->grid.ys * b->ctx[y]->grid.zs * (1 + b->grids[y].R);
     return wx > wy;
   });
-  std::vector<int2> items;
+  std::vector<int2>& items = b->items;
   for (int gi : order)
     for (int u = 0; u < b->grids[gi].units; ++u) items.push_back(make_int2(gi, u));
   b->total_items = (int)items.size();
@@ -681,7 +810,8 @@ int st3d_batch_create(uint32_t n, const st3d_grid_desc* grids, const st3d_opts* 
     cudaGetLastError();
     return cleanup(bfail(ST3D_ERR_UNSUPPORTED, "the batch kernel cannot be resident"));
   }
-  b->ctas = std::min(sm * per_sm, b->total_items);
+  b->max_ctas = sm * per_sm;
+  b->ctas = std::min(b->max_ctas, b->total_items);
   if (cudaMalloc(&b->d_grids, n * sizeof(BatchGrid)) != cudaSuccess ||
       cudaMalloc(&b->d_maps, maps.size() * sizeof(CUtensorMap)) != cudaSuccess ||
       cudaMalloc(&b->d_items, items.size() * sizeof(int2)) != cudaSuccess ||
@@ -769,23 +899,19 @@ int st3d_batch_iterate(st3d_batch* b, uint32_t steps, int schedule) {
     return ST3D_OK;
   }
   if (schedule == ST3D_BATCH_PERSISTENT) {
-    if ((rc = enqueue_persistent(b, steps)) != ST3D_OK) return rc;
+    if ((rc = enqueue_persistent(b, steps, b->d_items, b->total_items)) != ST3D_OK) return rc;
   } else {
     auto it = b->graphs.find(steps);
     if (it == b->graphs.end()) {
-      cudaGraph_t graph;
-      B_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-      rc = enqueue_persistent(b, steps);
-      cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+      st3d_batch::Graph graph;
+      const std::vector<char> none(b->ctx.size(), 0), alone = split_grids(b, steps);
+      rc = capture_graph(b, steps, alone, &graph);
+      // a GPU that cannot hold a multi-step launch: every grid in the queue
+      if (rc != ST3D_OK && alone != none) rc = capture_graph(b, steps, none, &graph);
       if (rc != ST3D_OK) return rc;
-      if (e != cudaSuccess) return set_error(ST3D_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-      cudaGraphExec_t exec;
-      e = cudaGraphInstantiate(&exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e != cudaSuccess) return set_error(ST3D_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
-      it = b->graphs.emplace(steps, exec).first;
+      it = b->graphs.emplace(steps, graph).first;
     }
-    B_CUDA(cudaGraphLaunch(it->second, b->stream));
+    B_CUDA(cudaGraphLaunch(it->second.exec, b->stream));
   }
   b->launches += steps;
   advance(b, steps);

@@ -209,6 +209,19 @@ size_t wave_words(int steps, int columns);
 cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
                         float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
                         uint32_t* dev_status, cudaStream_t stream);
+// The same with the buffer of u and the amplitudes read from device memory
+// when the launch runs (a captured launch that is replayed): u is in buffer
+// *ub_dev ^ flip, step m's amplitude at amps_dev[m * amp_stride].
+cudaError_t launch_wave_dev(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
+                            float* const* fld, const int* ub_dev, int flip, int steps, const Source& src,
+                            const float* amps_dev, int amp_stride, uint32_t* dev_status,
+                            cudaStream_t stream);
+// A context's multi-step wave plan (st3d_api.cu): makes it where the form
+// allows; the shape of a launch of `steps` steps with its estimated time.
+// plan_wave: false where single steps are the better choice (any = false) or
+// there is no such launch at all.
+void setup_wave(st3d_ctx* c, int sm_count);
+bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us = nullptr, bool any = false);
 
 // Reference layout (staging buffer) <-> library layout, element size eb.
 cudaError_t launch_ref_to_dev(int eb, const Layout& L, const RefGeom& R, const void* stage,

@@ -75,7 +75,8 @@ struct WaveArgs {
   Geom g;
   Coefs<float> cf;
   float* buf[2];
-  int ub0;               // buffer of U^n at the launch's first step
+  int ub0;               // buffer of U^n at the launch's first step, or, with ub_dev,
+  const int* ub_dev;     //   what *ub_dev is exclusive-ored with
   int steps;             // of this launch
   int T, S, Q, shift;    // levels, columns at work per level, columns, delay of a level
   int ntk;
@@ -85,6 +86,8 @@ struct WaveArgs {
   int src_i, src_j, src_k;
   uint64_t limit_ns;
   uint32_t* status;
+  const float* amps_dev;  // step m's amplitude at [m * amp_stride] instead of amps[m]
+  int amp_stride;
   float amps[kWaveSteps];
 };
 
@@ -183,6 +186,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x / a.S, s = blockIdx.x - t * a.S;
+  const int ub0 = a.ub_dev ? a.ub0 ^ __ldg(a.ub_dev) : a.ub0;
   if (threadIdx.x < NW + 1) stored[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -212,7 +216,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
       if (!u.live) continue;
       const int jt = u.q / a.ntk, kt = u.q - jt * a.ntk;
       const int k0 = kt * TK, j0 = jt * TJ;
-      const int ub = a.ub0 ^ (u.step & 1);
+      const int ub = ub0 ^ (u.step & 1);
       const CUtensorMap* um = ub ? &um1 : &um0;
       const CUtensorMap* vm = ub ? &vm0 : &vm1;
       const int nsteps = g.xs + 2 * R;
@@ -344,9 +348,9 @@ __global__ void __launch_bounds__(kWThreads, 1)
     const int k = kt * TK + 4 * kl;
     const int nsteps = g.xs + 2 * R;
     const bool row_ok = j < g.ys;
-    const int ub = a.ub0 ^ (u.step & 1);
+    const int ub = ub0 ^ (u.step & 1);
     float* vrow = a.buf[ub ^ 1] + g.org + (long long)j * g.sj + k;
-    const float amp = a.amps[u.step];
+    const float amp = a.amps_dev ? __ldg(a.amps_dev + (size_t)u.step * a.amp_stride) : a.amps[u.step];
     const int src_i = (j == a.src_j && (unsigned)(a.src_k - k) < 4u) ? a.src_i : -1;
     for (int n0 = 0; n0 < nsteps; n0 += QN) {
 #pragma unroll
@@ -479,16 +483,16 @@ int wave_blocks_per_sm(int points, bool narrow) {
 
 size_t wave_words(int steps, int columns) { return ((size_t)steps * columns + 1) * kWPad; }
 
-cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
-                        float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
-                        uint32_t* dev_status, cudaStream_t stream) {
+namespace {
+
+cudaError_t launch_any(const WavePlan& w, int points, WaveArgs& a, const Geom& g, const Coefs<float>& cf,
+                       float* const* fld, int steps, const Source& src, uint32_t* dev_status,
+                       cudaStream_t stream) {
   if (steps < 1 || steps > w.max_steps || w.T < 1 || w.S < 1) return cudaErrorInvalidValue;
-  WaveArgs a;
   a.g = g;
   a.cf = cf;
   a.buf[0] = fld[0];
   a.buf[1] = fld[1];
-  a.ub0 = ubuf;
   a.steps = steps;
   a.T = w.T;
   a.S = w.S;
@@ -503,7 +507,6 @@ cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coef
   a.src_k = src.k;
   a.limit_ns = w.limit_ns;
   a.status = dev_status;
-  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = n < steps ? amps[n] : 0.0f;
   cudaError_t e = cudaMemsetAsync(w.words, 0, wave_words(steps, a.Q) * sizeof(int), stream);
   if (e != cudaSuccess) return e;
   switch (points) {
@@ -512,6 +515,33 @@ cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coef
     case 25: return w.narrow ? launch_p<25, true>(w, a, stream) : launch_p<25, false>(w, a, stream);
     default: return cudaErrorInvalidValue;
   }
+}
+
+}  // namespace
+
+cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
+                        float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
+                        uint32_t* dev_status, cudaStream_t stream) {
+  WaveArgs a;
+  a.ub0 = ubuf;
+  a.ub_dev = nullptr;
+  a.amps_dev = nullptr;
+  a.amp_stride = 0;
+  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = n < steps ? amps[n] : 0.0f;
+  return launch_any(w, points, a, g, cf, fld, steps, src, dev_status, stream);
+}
+
+cudaError_t launch_wave_dev(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
+                            float* const* fld, const int* ub_dev, int flip, int steps, const Source& src,
+                            const float* amps_dev, int amp_stride, uint32_t* dev_status,
+                            cudaStream_t stream) {
+  WaveArgs a;
+  a.ub0 = flip;
+  a.ub_dev = ub_dev;
+  a.amps_dev = amps_dev;
+  a.amp_stride = amp_stride;
+  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = 0.0f;
+  return launch_any(w, points, a, g, cf, fld, steps, src, dev_status, stream);
 }
 
 }  // namespace st3d
