@@ -561,6 +561,13 @@ std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
     const double chunks = (double)G.units / G.ntjk;
     share[gi] = 0.6 * G.ntjk * (g.xs + chunks * 2 * c->R) / b->max_ctas;
     unit[gi] = 0.6 * (std::min<int>((int)g.xs, G.ichunk) + 2 * c->R);
+    if (c->brick.nbi > 0) {
+      own[gi] = 0.0;
+      for (uint32_t done = 0; done < steps; done += kWaveSteps)
+        own[gi] += brick_us(c->brick, c->R, (int)std::min(steps - done, (uint32_t)kWaveSteps));
+      order.push_back((int)gi);
+      continue;
+    }
     if (!c->wave) continue;
     double us = 0.0;
     WavePlan w;
@@ -612,13 +619,24 @@ int enqueue_alone(st3d_batch* b, uint32_t steps, const std::vector<char>& alone)
     Source src;
     src.i = c->opts.src_i; src.j = c->opts.src_j; src.k = c->opts.src_k;
     src.amp = 0.0f; src.amp_d = 0.0;
-    float* const fld[2] = {(float*)c->fld[0], (float*)c->fld[1]};
+    float* const fld[3] = {(float*)c->fld[0], (float*)c->fld[1], (float*)c->fld[2]};
     for (uint32_t done = 0; done < steps;) {
-      const uint32_t many = std::min(steps - done, (uint32_t)c->wave->max_steps);
-      WavePlan w;
-      if (!plan_wave(c, many, &w, nullptr, true)) return bfail(ST3D_ERR_CUDA, "no multi-step launch");
-      B_CUDA(launch_wave_dev(w, c->opts.points, c->G, c->cf32, fld, &b->d_grids[gi].cur0, (int)(done & 1),
-                             (int)many, src, b->d_amps + (size_t)done * n + gi, n, c->dev_status, b->stream));
+      const bool brick = c->brick.nbi > 0;
+      const uint32_t many = std::min(steps - done, (uint32_t)(brick ? kWaveSteps : c->wave->max_steps));
+      StepFeed feed;
+      feed.ub = (int)(done & 1);
+      feed.ub_dev = &b->d_grids[gi].cur0;
+      feed.amps_dev = b->d_amps + (size_t)done * n + gi;
+      feed.amp_stride = n;
+      if (brick) {
+        B_CUDA(launch_brick(c->brick, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed,
+                            c->brick_words, c->dev_status, b->stream));
+      } else {
+        WavePlan w;
+        if (!plan_wave(c, many, &w, nullptr, true)) return bfail(ST3D_ERR_CUDA, "no multi-step launch");
+        B_CUDA(launch_wave(w, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed, c->dev_status,
+                           b->stream));
+      }
       done += many;
     }
   }

@@ -74,6 +74,9 @@ struct st3d_ctx {
   size_t bytes = 0;
   // several wave steps a launch (st3d_kernels_wave.cu); nullptr: one a launch
   WavePlan* wave = nullptr;
+  // the same for grids that fit the SMs' shared memory (st3d_kernels_brick.cu)
+  st3d::BrickPlan brick;  // nbi = 0: none
+  int* brick_words = nullptr;  // part of `scratch`
   // the streamed drop-in call (st3d_stream.cu): its queues, counters and
   // amplitudes on the device, and their host copies (kept until the next call)
   void* stream_buf = nullptr;

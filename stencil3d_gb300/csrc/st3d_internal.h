@@ -206,16 +206,36 @@ int wave_tile_cols(bool narrow);
 int wave_blocks_per_sm(int points, bool narrow);
 // Words of device memory a launch of that many steps keeps its progress in.
 size_t wave_words(int steps, int columns);
+// Where a multi-step launch takes the buffer of u and the source amplitudes
+// from: the host's values now, or device memory when it runs (a captured
+// launch that is replayed): u is in buffer *ub_dev ^ ub, step m's amplitude at
+// amps_dev[m * amp_stride].
+struct StepFeed {
+  int ub = 0;
+  const int* ub_dev = nullptr;
+  const float* amps = nullptr;      // host, one per step
+  const float* amps_dev = nullptr;
+  int amp_stride = 0;
+};
+// fld: the u/v pair and s.
 cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
-                        float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
+                        float* const* fld, int steps, const Source& src, const StepFeed& feed,
                         uint32_t* dev_status, cudaStream_t stream);
-// The same with the buffer of u and the amplitudes read from device memory
-// when the launch runs (a captured launch that is replayed): u is in buffer
-// *ub_dev ^ flip, step m's amplitude at amps_dev[m * amp_stride].
-cudaError_t launch_wave_dev(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
-                            float* const* fld, const int* ub_dev, int flip, int steps, const Source& src,
-                            const float* amps_dev, int amp_stride, uint32_t* dev_status,
-                            cudaStream_t stream);
+
+// Many FP32 wave steps of a small grid in one launch, its fields in shared
+// memory (st3d_kernels_brick.cu).
+struct BrickPlan {
+  int bi = 0, bj = 0, nbi = 0, nbj = 0;  // brick extents, bricks along i and j
+  int zq = 0, pitch = 0;                 // quads of a row, floats of a row in shared memory
+};
+constexpr int kBricks = 160;  // at most (one an SM)
+size_t brick_words(int bricks);
+bool plan_brick(const Geom& g, int R, int sms, size_t max_smem, BrickPlan* best);
+// Estimated time of a launch, microseconds.
+double brick_us(const BrickPlan& p, int R, int steps);
+cudaError_t launch_brick(const BrickPlan& p, int points, const Geom& g, const Coefs<float>& cf,
+                         float* const* fld, int steps, const Source& src, const StepFeed& feed, int* words,
+                         uint32_t* dev_status, cudaStream_t stream);
 // A context's multi-step wave plan (st3d_api.cu): makes it where the form
 // allows; the shape of a launch of `steps` steps with its estimated time.
 // plan_wave: false where single steps are the better choice (any = false) or

@@ -483,16 +483,20 @@ int wave_blocks_per_sm(int points, bool narrow) {
 
 size_t wave_words(int steps, int columns) { return ((size_t)steps * columns + 1) * kWPad; }
 
-namespace {
-
-cudaError_t launch_any(const WavePlan& w, int points, WaveArgs& a, const Geom& g, const Coefs<float>& cf,
-                       float* const* fld, int steps, const Source& src, uint32_t* dev_status,
-                       cudaStream_t stream) {
+cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
+                        float* const* fld, int steps, const Source& src, const StepFeed& feed,
+                        uint32_t* dev_status, cudaStream_t stream) {
   if (steps < 1 || steps > w.max_steps || w.T < 1 || w.S < 1) return cudaErrorInvalidValue;
+  WaveArgs a;
   a.g = g;
   a.cf = cf;
   a.buf[0] = fld[0];
   a.buf[1] = fld[1];
+  a.ub0 = feed.ub;
+  a.ub_dev = feed.ub_dev;
+  a.amps_dev = feed.amps_dev;
+  a.amp_stride = feed.amp_stride;
+  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = n < steps && feed.amps ? feed.amps[n] : 0.0f;
   a.steps = steps;
   a.T = w.T;
   a.S = w.S;
@@ -515,33 +519,6 @@ cudaError_t launch_any(const WavePlan& w, int points, WaveArgs& a, const Geom& g
     case 25: return w.narrow ? launch_p<25, true>(w, a, stream) : launch_p<25, false>(w, a, stream);
     default: return cudaErrorInvalidValue;
   }
-}
-
-}  // namespace
-
-cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
-                        float* const* fld, int ubuf, int steps, const Source& src, const float* amps,
-                        uint32_t* dev_status, cudaStream_t stream) {
-  WaveArgs a;
-  a.ub0 = ubuf;
-  a.ub_dev = nullptr;
-  a.amps_dev = nullptr;
-  a.amp_stride = 0;
-  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = n < steps ? amps[n] : 0.0f;
-  return launch_any(w, points, a, g, cf, fld, steps, src, dev_status, stream);
-}
-
-cudaError_t launch_wave_dev(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
-                            float* const* fld, const int* ub_dev, int flip, int steps, const Source& src,
-                            const float* amps_dev, int amp_stride, uint32_t* dev_status,
-                            cudaStream_t stream) {
-  WaveArgs a;
-  a.ub0 = flip;
-  a.ub_dev = ub_dev;
-  a.amps_dev = amps_dev;
-  a.amp_stride = amp_stride;
-  for (int n = 0; n < kWaveSteps; ++n) a.amps[n] = 0.0f;
-  return launch_any(w, points, a, g, cf, fld, steps, src, dev_status, stream);
 }
 
 }  // namespace st3d
