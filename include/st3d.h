@@ -235,7 +235,8 @@ int st3d_transfer(st3d_ctx* dst, st3d_ctx* src);
  * halo).  One contiguous copy per field through a staging buffer the context
  * allocates on first use (the size of one host array).  The arrays may be
  * host memory or device memory of the context's device (st3d_download
- * likewise).  Resets the mode W step clock to 0. */
+ * likewise).  Host arrays may be written again when the call returns; device
+ * arrays are read in stream order.  Resets the mode W step clock to 0. */
 int st3d_upload(st3d_ctx* ctx, const void* v, const void* s, const void* u);
 /* Copy interior points out: the host arrays' halo planes and rows are not
  * written, as the reference never writes halos; the k-halo points between

@@ -1202,6 +1202,74 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   return ST3D_OK;
 }
 
+// st3d_upload without its wait for pinned arrays.
+int upload_fields(st3d_ctx* c, const void* v, const void* s, const void* u) {
+  int rc;
+  if (c->delta) {
+    c->step = 0;
+    if ((rc = ensure_stage(c, 2)) != ST3D_OK) return rc;
+    if (u || v) {
+      if (!(u && v) && !c->pair_valid && (rc = delta_rebuild_pair(c)) != ST3D_OK) return rc;
+      c->pair_valid = false;
+      if (u)
+        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), u, host_array_bytes(c), cudaMemcpyDefault,
+                                  c->stream));
+      if (v)
+        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 1), v, host_array_bytes(c), cudaMemcpyDefault,
+                                  c->stream));
+      if ((rc = delta_encode_pair(c, u != nullptr)) != ST3D_OK) return rc;
+      if (u) c->has_u = true;
+      if (v) c->has_v = true;
+    }
+    if (s) {
+      c->pair_valid = false;  // s passes through slot 0, unless it is a device array
+      const float* src = stage_slot(c, 0);
+      if (device_view(c, s, host_array_bytes(c)))
+        src = static_cast<const float*>(s);
+      else
+        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), s, host_array_bytes(c), cudaMemcpyDefault,
+                                  c->stream));
+      if ((rc = encode_staged16(c, src, nullptr, c->fld[2], M_s(c), E_s(c), "s")) !=
+          ST3D_OK)
+        return rc;
+      c->has_s = true;
+    }
+    return ST3D_OK;
+  }
+  if (c->f16) {
+    c->step = 0;
+    if (u) {
+      if ((rc = upload_field16(c, 0, u)) != ST3D_OK) return rc;
+      c->has_u = true;
+    }
+    if (v) {
+      if ((rc = upload_field16(c, 1, v)) != ST3D_OK) return rc;
+      c->has_v = true;
+    }
+    if (s) {
+      if ((rc = upload_field16(c, 2, s)) != ST3D_OK) return rc;
+      c->has_s = true;
+    }
+    ST3D_CUDA(cudaMemsetAsync(M_level(c, (long long)c->lvl + 1), 0, c->grid.xs * sizeof(uint32_t), c->stream));
+    ST3D_CUDA(cudaMemsetAsync(M_level(c, (long long)c->lvl + 2), 0, c->grid.xs * sizeof(uint32_t), c->stream));
+    return ST3D_OK;
+  }
+  if (u) {
+    if ((rc = upload_field(c, u_ptr(c), u)) != ST3D_OK) return rc;
+    c->has_u = true;
+  }
+  if (v) {
+    if ((rc = upload_field(c, v_ptr(c), v)) != ST3D_OK) return rc;
+    c->has_v = true;
+  }
+  if (s) {
+    if ((rc = upload_field(c, c->fld[2], s)) != ST3D_OK) return rc;
+    c->has_s = true;
+  }
+  c->step = 0;
+  return ST3D_OK;
+}
+
 int check_device_status(st3d_ctx* c) {
   uint32_t st = 0;
   ST3D_CUDA(cudaMemcpyAsync(&st, c->dev_status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
@@ -1685,69 +1753,23 @@ int st3d_get_stream(const st3d_ctx* c, void** s) {
 int st3d_upload(st3d_ctx* c, const void* v, const void* s, const void* u) {
   if (!c) return fail(ST3D_ERR_INVALID, "null context");
   DeviceScope scope(c->device);
-  int rc;
-  if (c->delta) {
-    c->step = 0;
-    if ((rc = ensure_stage(c, 2)) != ST3D_OK) return rc;
-    if (u || v) {
-      if (!(u && v) && !c->pair_valid && (rc = delta_rebuild_pair(c)) != ST3D_OK) return rc;
-      c->pair_valid = false;
-      if (u)
-        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), u, host_array_bytes(c), cudaMemcpyDefault,
-                                  c->stream));
-      if (v)
-        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 1), v, host_array_bytes(c), cudaMemcpyDefault,
-                                  c->stream));
-      if ((rc = delta_encode_pair(c, u != nullptr)) != ST3D_OK) return rc;
-      if (u) c->has_u = true;
-      if (v) c->has_v = true;
+  int rc = upload_fields(c, v, s, u);
+  if (rc != ST3D_OK) return rc;
+  // pinned host arrays are read while the stream runs: wait, so that the
+  // caller may write them again (pageable ones have been copied by now)
+  for (const void* p : {v, s, u}) {
+    cudaPointerAttributes at;
+    if (!p || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
     }
-    if (s) {
-      c->pair_valid = false;  // s passes through slot 0, unless it is a device array
-      const float* src = stage_slot(c, 0);
-      if (device_view(c, s, host_array_bytes(c)))
-        src = static_cast<const float*>(s);
-      else
-        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), s, host_array_bytes(c), cudaMemcpyDefault,
-                                  c->stream));
-      if ((rc = encode_staged16(c, src, nullptr, c->fld[2], M_s(c), E_s(c), "s")) !=
-          ST3D_OK)
-        return rc;
-      c->has_s = true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (at.type == cudaMemoryTypeHost && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess &&
+        cap == cudaStreamCaptureStatusNone) {
+      ST3D_CUDA(cudaStreamSynchronize(c->stream));
+      break;
     }
-    return ST3D_OK;
   }
-  if (c->f16) {
-    c->step = 0;
-    if (u) {
-      if ((rc = upload_field16(c, 0, u)) != ST3D_OK) return rc;
-      c->has_u = true;
-    }
-    if (v) {
-      if ((rc = upload_field16(c, 1, v)) != ST3D_OK) return rc;
-      c->has_v = true;
-    }
-    if (s) {
-      if ((rc = upload_field16(c, 2, s)) != ST3D_OK) return rc;
-      c->has_s = true;
-    }
-    ST3D_CUDA(cudaMemsetAsync(M_level(c, (long long)c->lvl + 1), 0, c->grid.xs * sizeof(uint32_t), c->stream));
-    ST3D_CUDA(cudaMemsetAsync(M_level(c, (long long)c->lvl + 2), 0, c->grid.xs * sizeof(uint32_t), c->stream));
-    return ST3D_OK;
-  }
-  if (u) {
-    if ((rc = upload_field(c, u_ptr(c), u)) != ST3D_OK) return rc;
-    c->has_u = true;
-  }
-  if (v) {
-    if ((rc = upload_field(c, v_ptr(c), v)) != ST3D_OK) return rc;
-    c->has_v = true;
-  }
-  if (s) {
-    if ((rc = upload_field(c, c->fld[2], s)) != ST3D_OK) return rc;
-    c->has_s = true;
-  }
-  c->step = 0;
   return ST3D_OK;
 }
 
@@ -1945,7 +1967,7 @@ int st3d_iterate_host(st3d_ctx* c, void* v, const void* s, void* u, uint32_t ite
   int rc = iterate_host_streamed(c, v, s, u, iterations, &streamed);
   if (rc != ST3D_OK) return rc;
   if (streamed) return st3d_synchronize(c);
-  rc = st3d_upload(c, v, s, u);
+  rc = upload_fields(c, v, s, u);
   if (rc == ST3D_OK) rc = st3d_iterate(c, iterations);
   if (rc == ST3D_OK)
     rc = st3d_download(c, v, c->opts.mode == ST3D_MODE_WAVE ? u : nullptr);
