@@ -925,10 +925,13 @@ void setup_wave(st3d_ctx* c, int sm_count) {
   for (int n = 0; n < 2 && ok == ST3D_OK; ++n) {
     WaveShape& sh = w->shape[n];
     const int tj = wave_tile_rows(n), tk = wave_tile_cols(n);
-    const long long ntk = ((long long)c->L.zs + tk - 1) / tk, Q = ((long long)c->L.ys + tj - 1) / tj * ntk;
+    const long long ntk = ((long long)c->L.zs + tk - 1) / tk, ntj = ((long long)c->L.ys + tj - 1) / tj;
+    // columns with the rows that the skew of the levels adds
+    const long long Q = (ntj + (kWaveLevels - 1) * c->R / tj + 1) * ntk;
     if (Q > (1 << 18)) ok = ST3D_ERR_UNSUPPORTED;
+    sh.tj = tj;
     sh.ntk = (int)ntk;
-    sh.Q = (int)Q;
+    sh.ntj = (int)ntj;
     most = std::max(most, Q);
     for (int f = 0; f < 3 && ok == ST3D_OK; ++f) {
       if (f < 2)
@@ -939,6 +942,7 @@ void setup_wave(st3d_ctx* c, int sm_count) {
   if (ok == ST3D_OK) {
     // a progress word per step and column: 8 MB at most, but 8 steps
     w->max_steps = (int)std::min<long long>(kWaveSteps, std::max(8LL, (1LL << 16) / most));
+    w->max_columns = (int)most;
     w->words_n = wave_words(w->max_steps, (int)most);
     if (cudaMalloc(&w->words, w->words_n * sizeof(int)) != cudaSuccess) ok = ST3D_ERR_NOMEM;
   }
@@ -950,28 +954,59 @@ void setup_wave(st3d_ctx* c, int sm_count) {
   c->wave = w;  // its words, like the other scratch, are not counted in c->bytes
 }
 
+// Estimated time of one step a launch (see plan_wave).
+double single_step_us(const st3d_ctx* c) {
+  const TmaPlan& p = *c->tma;
+  const bool big = 12.0 * c->grid.xs * c->grid.ys * c->grid.zs >= 1.0e8;
+  const double fill = (double)c->L.ys * c->L.zs / ((double)p.ntj * p.tj * p.ntk * kTmaTK);
+  return 3.5 + (double)((p.units + p.grid - 1) / p.grid) * (p.ichunk + c->R) *
+                   (big ? 0.76 * (0.2 + 0.8 * fill) : 0.5);
+}
+
+// Lays T levels of the tile shape `nar` out on `ctas` CTAs; false where the
+// columns or levels are more than the progress words hold.
+bool wave_layout(WavePlan* w, int nar, int T, int ctas, const Layout& L, int R) {
+  const WaveShape& sh = w->shape[nar];
+  w->narrow = nar;
+  w->T = T;
+  w->skew = w->shift = 0;
+  w->Q = sh.ntj * sh.ntk;
+  if (w->Q > ctas / T) {
+    // several turns: each level R rows lower and one column later
+    w->skew = R;
+    w->shift = 1;
+    w->Q = (int)(((long long)L.ys + (T - 1) * R + sh.tj - 1) / sh.tj) * sh.ntk;
+  }
+  w->S = std::min(w->Q, ctas / T);
+  return T <= kWaveLevels && w->S >= 1 && w->Q <= w->max_columns;
+}
+// Columns one CTA takes one after the other for n steps.
+double wave_turns(const WavePlan& w, int n) {
+  const long long passes = (n + w.T - 1) / w.T;
+  return (double)((passes * w.Q + (long long)(w.T - 1) * w.shift + w.S - 1) / w.S);
+}
+
 // The shape of a launch of `steps` wave steps; false: one step a launch is
 // the better choice.  The times compared, in microseconds, are fitted to
 // measurements on a GB300 (FP32, 20 to 40 steps, device time):
 //   several steps: a CTA takes a plane of its column in 0.34 / 0.38 / 0.60 us
 //     (7 / 13 / 25 points) while the three fields fit L2, 0.47 / 0.48 / 0.62
-//     up to 300 MB and 0.55 / 0.56 / 0.62 beyond, where 4 and 5 levels are
-//     best (7 points 512^3, Gpts/s with 2 / 3 / 4 / 5 / 6 levels: 496 / 521 /
-//     549 / 567 / 506; 25 points, 1024^2 planes: 449 / 436 / 458 / 447 / 375);
+//     up to 300 MB and 0.55 / 0.56 / 0.62 beyond, where 4 and 5 levels are best
+//     (Gpts/s with 2 / 3 / 4 / 5 / 6 levels: 7 points, 1024^2 planes 484 / 518 /
+//     571 / 589 / 516; 25 points 443 / 434 / 463 / 463 / 381);
 //     several turns below 300 MB 15 % more (13 points 301 x 187 x 423: 48
-//     columns at once in 3 levels 1044 us, 38 at a time in 4 levels 1160),
-//     30 % with more than 5 levels; a column whose next level waits for the
-//     next turn finds its planes gone from L2 (shift of S columns: 25 points
-//     343 x 341 x 1412, 23 of 76: 2937 us against 2539 for single steps);
-//     a level starts 6.5 us after the one before; 32 x 64 tiles take 5 % more
-//     a plane (25 points, 1024^2 planes 431 against 458 Gpts/s) and pay off
-//     where they pad less (528^3: 417 against 399);
+//     columns at once in 3 levels 1058 us, 38 at a time in 4 levels 1160),
+//     30 % with more than 5 levels;
+//     a level starts 6 + R us after the one before; 32 x 64 tiles take 5 % more
+//     a plane and pay off where they pad less (25 points 528^3: 420 against
+//     380 Gpts/s);
 //   one step a launch: its units' planes (with R warm-up planes) at 0.76 us
 //     where the tiles are full (padding costs no HBM bytes), 0.5 in L2, and
 //     3.5 us a launch.
 // Measured (one step a launch -> several): 7 points 256^3 x 20 937 -> 590 us,
-// 13 points 301 x 187 x 423 x 20 1413 -> 1044, 25 points 528^3 x 40 15930 ->
-// 14113; 7 points 128^3 x 20 stays at one (145 against 159).
+// 13 points 301 x 187 x 423 x 20 1413 -> 1058, 25 points 528^3 x 40 15969 ->
+// 14009, 1024^3 x 20 54748 -> 45771; 7 points 128^3 x 20 stays at one (145
+// against 159).
 bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, bool any) {
   if (!c->wave || steps < 2) return false;
   const int n = (int)steps, R = c->R, xs = (int)c->L.xs;
@@ -981,42 +1016,28 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
   const double tau = plane_us[R == 1 ? 0 : R == 2 ? 1 : 2][size];
   static const double levels[7] = {0.0, 0.0, 1.08, 1.05, 1.0, 1.0, 1.18};
   double best = 1e300;
-  int best_T = 0, best_n = 0;
+  int best_T = 0;
   for (int nar = 0; nar < 2; ++nar) {
-    const int Q = c->wave->shape[nar].Q, ntk = c->wave->shape[nar].ntk;
     for (int T = 2; T <= std::min({n, c->wave->ctas, 24}); ++T) {
-      const int S = std::min(Q, c->wave->ctas / T);
-      const long long shift = Q <= S ? 0 : ntk;
-      // every dependency at the same or an earlier place of the sequence
-      if (shift && Q < ntk + (T - 1) * shift) break;
-      const long long passes = (n + T - 1) / T, turns = (passes * Q + (T - 1) * shift + S - 1) / S;
-      const double us = turns * (xs + 2.0 * R) * tau * (nar ? 1.05 : 1.0) *
-                            (size == 2 ? levels[std::min(T, 6)] : !shift ? 1.0 : T > 5 ? 1.3 : 1.15) *
-                            (1.0 + 0.4 * std::max(0.0, (double)shift / S - 0.2)) +
-                        6.5 * (T - 1) + 12.0;
+      WavePlan v = *c->wave;
+      if (!wave_layout(&v, nar, T, v.ctas, c->L, R)) break;
+      const double us = wave_turns(v, n) * (xs + 2.0 * R) * tau * (nar ? 1.05 : 1.0) *
+                            (size == 2 ? levels[std::min(T, 6)] : !v.shift ? 1.0 : T > 5 ? 1.3 : 1.15) +
+                        (6.0 + R) * (T - 1) + 12.0;
       if (us < best) {
         best = us;
         best_T = T;
-        best_n = nar;
+        *w = v;
       }
     }
   }
-  const TmaPlan& p = *c->tma;
-  const double fill = (double)c->L.ys * c->L.zs / ((double)p.ntj * p.tj * p.ntk * kTmaTK);
-  const double one = 3.5 + (double)((p.units + p.grid - 1) / p.grid) * (p.ichunk + R) *
-                               (size ? 0.76 * (0.2 + 0.8 * fill) : 0.5);
-  if (!best_T || (!any && best > 0.93 * n * one)) return false;
+  if (!best_T || (!any && best > 0.93 * n * single_step_us(c))) return false;
   if (est_us) *est_us = best;
-  *w = *c->wave;
-  w->narrow = best_n;
-  w->T = best_T;
-  const int Q = w->shape[best_n].Q;
-  w->S = std::min(Q, w->ctas / best_T);
-  w->shift = Q <= w->S ? 0 : w->shape[best_n].ntk;
   // beyond R + 1 planes, or the slowest of two neighbours could wait for the
-  // other; unbounded (7 points 256^3, 201 MB: 590 against 618 us) where L2
+  // other (16 / 20 / 26 / 32 planes, Gpts/s: 25 points, 1024^2 planes 439 / 467 /
+  // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497); unbounded (7 points 256^3, 201 MB: 590 against 618 us) where L2
   // has room (13 points 301 x 187 x 423, 286 MB: 1149 against 1044)
-  w->couple = bytes > 2.4e8 ? 18 + 2 * R : 1 << 28;
+  w->couple = bytes > 2.4e8 ? kWaveCouple : 1 << 28;
   w->limit_ns = 4000000000ull + (uint64_t)(bytes / 12.0 * n / 2.5);
   return true;
 }
@@ -1024,6 +1045,82 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
 }  // namespace st3d
 
 namespace {
+
+// The streamed drop-in call of the wave form as one launch of the multi-step
+// kernel with its transfer CTAs: device views of the pinned host arrays.  Takes
+// as many levels as steps where the CTAs allow, so that columns reach their last
+// step in the order they came in (25 points 512^3, 20 steps in 20 / 10 / 7
+// levels: 12.9 / 15.6 / 17.9 ms; chunks of planes, st3d_stream.cu, 15.9).
+// *done = false where another way is the only one.
+int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32_t iterations, bool* done) {
+  const int n = (int)std::min<uint32_t>(iterations, 1u << 20), R = c->R, xs = (int)c->L.xs;
+  const st3d_grid_desc& gd = c->grid;
+  WavePlan w = *c->wave;
+  if (n < 4 || n > w.max_steps || w.ctas < 64) return ST3D_OK;
+  WaveXfer x;
+  // 25 points 512^3, 20 steps, with 12 / 16 / 20 / 24 upload and 12 download
+  // CTAs: 13.8 / 12.9 / 12.3 / 12.6 ms a call
+  x.n_up = 20;
+  x.n_down = 12;
+  x.planes = 16;
+  const int ctas = w.ctas - x.n_up - x.n_down;
+  double best = 1e300;
+  for (int nar = 0; nar < 2; ++nar)
+    for (int T = 2; T <= std::min({n, ctas, kWaveLevels}); ++T) {
+      WavePlan v = w;
+      if (!wave_layout(&v, nar, T, ctas, c->L, R)) break;
+      const double us = wave_turns(v, n) * (xs + 2 * R) * (nar ? 1.05 : 1.0) * (n > T ? 1.3 : 1.0);
+      if (us < best) {
+        best = us;
+        w = v;
+      }
+    }
+  if (best > 1e299) return ST3D_OK;
+  w.couple = kWaveCouple;
+  x.R = ref_geom(gd);
+  x.s = static_cast<float*>(c->fld[2]);
+  x.hin[0] = hu;
+  x.hin[1] = hv;
+  x.hin[2] = hs;
+  x.hout[0] = hv;
+  x.hout[1] = hu;
+  x.hx = gd.xh < 4 ? (int)gd.xh : 4;
+  x.hy = gd.yh < 4 ? (int)gd.yh : 4;
+  x.hz = (int)gd.zh;
+  const bool aligned = (reinterpret_cast<uintptr_t>(hu) | reinterpret_cast<uintptr_t>(hv) |
+                        reinterpret_cast<uintptr_t>(hs)) % 16 == 0;
+  x.vec = aligned && x.R.jmult % 4 == 0 && gd.zh % 4 == 0 && gd.zs % 4 == 0;
+  // far beyond any run that makes progress: the steps at 2.5 Gpts/s, the
+  // transfers at 5 GB/s
+  const double pts = (double)gd.xs * gd.ys * gd.zs;
+  w.limit_ns = 4000000000ull + (uint64_t)(pts * n / 2.5 + 5.0 * host_array_bytes(c) / 5.0);
+  std::vector<float> amps(n, 0.0f);
+  Source src;
+  src.i = c->opts.src_i; src.j = c->opts.src_j; src.k = c->opts.src_k;
+  src.amp = 0.0f; src.amp_d = 0.0;
+  if (src.i >= 0)
+    for (int m = 0; m < n; ++m)
+      amps[m] = (float)st3d_ricker((double)m * c->opts.dt, c->opts.src_f, c->opts.src_t0);
+  float* const fld[3] = {(float*)c->fld[0], (float*)c->fld[1], (float*)c->fld[2]};
+  StepFeed feed;
+  feed.ub = c->ub;
+  feed.amps = amps.data();
+  cudaError_t e = launch_wave(w, c->opts.points, c->G, c->cf32, fld, n, src, feed, c->dev_status, c->stream, &x);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return ST3D_OK;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "streamed call launch");
+  c->has_u = c->has_v = c->has_s = true;
+  c->pair_valid = false;
+  c->step = (uint64_t)n;
+  c->lvl += (uint64_t)n;
+  c->launches += 1;
+  if (n & 1) std::swap(c->ub, c->vb);
+  c->host_path = ST3D_HOST_STREAMED;
+  *done = true;
+  return ST3D_OK;
+}
 
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and
 // download in one cooperative launch.  *done = false (and nothing enqueued)
@@ -1043,6 +1140,10 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   const float* hs = static_cast<const float*>(direct_view(s, hbytes));
   const float* hu = static_cast<const float*>(direct_view(u, hbytes));
   if (!hv || !hs || !hu) return ST3D_OK;
+  if (c->wave) {
+    const int rc = iterate_host_wave(c, const_cast<float*>(hv), hs, const_cast<float*>(hu), iterations, done);
+    if (rc != ST3D_OK || *done) return rc;
+  }
   int coop = 0, sm = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
   cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, c->device);

@@ -199,6 +199,8 @@ bool tma_config_supported(int tj, int nv);
 int tma_blocks_per_sm(int points, int mode, int tj, int nv, size_t smem);
 
 // Many FP32 wave steps in one launch (st3d_kernels_wave.cu).
+constexpr int kWaveCouple = 20;  // planes a column of level 0 may be ahead of its neighbours
+constexpr int kWaveLevels = 32;  // levels of one launch at most
 constexpr int kWaveSteps = 256;  // steps of one launch at most (the amplitudes are kernel arguments)
 struct WavePlan;
 int wave_tile_rows(bool narrow);
@@ -217,10 +219,20 @@ struct StepFeed {
   const float* amps_dev = nullptr;
   int amp_stride = 0;
 };
+// The transfers of a streamed drop-in call: upload and download CTAs (0: none),
+// host arrays u, v, s in and v, u out, planes of an item, the halo moved.
+struct WaveXfer {
+  int n_up = 0, n_down = 0, planes = 0;
+  RefGeom R;
+  float* s = nullptr;
+  const float* hin[3] = {nullptr, nullptr, nullptr};
+  float* hout[2] = {nullptr, nullptr};
+  int hx = 0, hy = 0, hz = 0, vec = 0;
+};
 // fld: the u/v pair and s.
 cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
                         float* const* fld, int steps, const Source& src, const StepFeed& feed,
-                        uint32_t* dev_status, cudaStream_t stream);
+                        uint32_t* dev_status, cudaStream_t stream, const WaveXfer* xfer = nullptr);
 
 // Many FP32 wave steps of a small grid in one launch, its fields in shared
 // memory (st3d_kernels_brick.cu).

@@ -14,16 +14,18 @@
 // the one-step kernel's result).
 //
 // Order.  Level t runs the columns q = 0, 1, ... of pass 0, 1, ... as one
-// sequence, x = p*Q + q, `shift` columns late per level (a row of tiles, so
-// that the columns beside a column are under way a level below; 0 when all
-// columns are at work at once): CTA (t, s) takes x + t*shift = s, s + S,
-// s + 2S, ...  Step n of column q at plane i reads U^n up to plane i + R of
-// the column and its four neighbours (the cross needs no corner) and
-// overwrites U^{n-1}, which step n - 1 of the same five columns read; both
-// are safe once those five have stored plane i + R of step n - 1.  Every
-// dependency is on the step before at the same or an earlier place of the
-// sequence, and the launch is cooperative (all CTAs resident), so every wait
-// ends.
+// sequence, x = p*Q + q, `shift` columns late per level: CTA (t, s) takes
+// x + t*shift = s, s + S, s + 2S, ...  A tile's rows lie `skew` rows lower at
+// each level, so with skew = R a column needs nothing of the row of tiles after
+// its own and a level may follow one column behind (shift = 1, the neighbour
+// along k).  When all columns are at work at once there is no skew and no shift.
+// Step n of a column at plane i reads U^n up to plane i + R of the tiles that
+// hold its rows with R either side and of those beside it along k (the cross
+// needs no corner), and overwrites U^{n-1}, which step n - 1 of the same tiles
+// read; both are safe once those tiles have stored plane i + R of step n - 1.
+// A step waits for the step before only, and each CTA takes its units pass by
+// pass: by induction over (pass, level) every wait ends, the launch being
+// cooperative (all CTAs resident).
 //
 // What bounds it is whether L2 (126 MB, 20 TB/s read) still holds a plane
 // when the next level comes for it.  The columns of level 0 depend on nothing
@@ -31,7 +33,10 @@
 // lag grows, and past about 20 us of lag at 430 Gpts/s the planes are gone
 // before they are read (7 points, 1024^2 planes: 11.5 bytes read from HBM a
 // point and step).  So level 0 is held to `couple` planes of its neighbours:
-// 7 points 512^3 437 -> 568 Gpts/s, 25 points 1024^2 planes 392 -> 463.  The
+// 7 points 512^3 437 -> 568 Gpts/s, 25 points 1024^2 planes 392 -> 463; the skew
+// (before it a level followed a row of tiles behind, and a fifth of the columns
+// found their planes gone at the next turn) 1024^3 at 7 / 25 points 528 -> 576 and
+// 458 -> 469.  The
 // columns' progress words lie 128 bytes apart: packed, all CTAs polled one L2
 // slice and every tile load met that queue (7 points 256^3: 1150 us against
 // 590; 25 points 528^3: 18.0 ms against 15.2).  The limit above that is
@@ -49,6 +54,16 @@
 //     may be loaded in shared memory, where the producer finds them.
 // Every wait ends: past `limit_ns` it sets the status word and an abort word
 // that all other waits look at.
+//
+// The streamed drop-in call (pinned host arrays, STREAM = true) runs as the same
+// pipeline with its transfers: `n_up` more CTAs copy u, v and s in, a row of
+// tiles (slab) after the other over all planes, `n_down` copy the last two
+// levels of a slab out once its columns have stored them.  A column's first step
+// waits until its slab and the two beside it are in; everything later follows
+// by the columns' own order.  With as many levels as steps the first slabs leave
+// while the last are still coming.
+#include <type_traits>
+
 #include "st3d_internal.h"
 #include "st3d_p4.cuh"
 #include "st3d_tma.cuh"
@@ -79,6 +94,7 @@ struct WaveArgs {
   const int* ub_dev;     //   what *ub_dev is exclusive-ored with
   int steps;             // of this launch
   int T, S, Q, shift;    // levels, columns at work per level, columns, delay of a level
+  int skew;              // rows a tile lies lower at each level
   int ntk;
   int couple;            // level 0: planes a column may be ahead of its neighbours
   int* prog;             // [step][Q], kWPad apart: planes stored
@@ -89,6 +105,9 @@ struct WaveArgs {
   const float* amps_dev;  // step m's amplitude at [m * amp_stride] instead of amps[m]
   int amp_stride;
   float amps[kWaveSteps];
+  WaveXfer x;
+  int* up_cnt;           // per slab (kWPad apart): items copied in
+  int* heads;            // upload and download queue
 };
 
 __device__ __forceinline__ void w_st_release(int* p, int v) {
@@ -140,8 +159,11 @@ __device__ __forceinline__ bool wait_bar(const WaveArgs& a, uint64_t* bar, uint3
 // The CTA's units in order: unit(r) is its r-th turn.  False past the end.
 struct Turn {
   int q, step, pass;
-  bool live;  // a column to work on (a level waits `shift` columns at first, and skips steps past the last)
+  int jt, kt, j0;  // tile and its first row (may lie outside the grid)
+  bool live;  // a column to work on (a level waits `shift` columns at first, skips steps past
+              // the last and tiles without a row of the grid)
 };
+template <int TJ>
 __device__ __forceinline__ bool turn(const WaveArgs& a, int t, int s, int r, Turn* u) {
   const int x = r * a.S + s - t * a.shift;
   u->live = false;
@@ -150,11 +172,131 @@ __device__ __forceinline__ bool turn(const WaveArgs& a, int t, int s, int r, Tur
   u->q = x - u->pass * a.Q;
   if ((long long)u->pass * a.T >= a.steps) return false;
   u->step = u->pass * a.T + t;
-  u->live = u->step < a.steps;
+  u->jt = u->q / a.ntk;
+  u->kt = u->q - u->jt * a.ntk;
+  u->j0 = u->jt * TJ - a.skew * t;
+  u->live = u->step < a.steps && u->j0 < a.g.ys && u->j0 + TJ > 0;
   return true;
 }
 
-template <int P, bool NARROW>
+__device__ __forceinline__ void w_red_release(int* p, int v) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Rows [ja, jb) of plane i between the host span and the field: one contiguous
+// run on the host side, whole words of W points, warps on 128-byte lines.
+template <int W, bool UP>
+__device__ __forceinline__ void copy_rows(const WaveArgs& a, float* dev, float* host, int i, int ja, int jb) {
+  using V = typename std::conditional<W == 4, float4, float>::type;
+  const WaveXfer& x = a.x;
+  const int kv = (x.R.zs + 2 * x.hz) / W;
+  const int n = (jb - ja) * kv;
+  V* span = reinterpret_cast<V*>(host + x.R.ijk_ofs + (long long)i * x.R.imult + (long long)ja * x.R.jmult - x.hz);
+  V* rows = reinterpret_cast<V*>(dev + a.g.org + (long long)i * a.g.si + (long long)ja * a.g.sj - x.hz);
+  const int pitch = (int)(a.g.sj / W);
+  const int shift = (int)((reinterpret_cast<uintptr_t>(span) / sizeof(V)) % (128 / sizeof(V)));
+  constexpr int UN = W == 4 ? 4 : 8;
+  for (int y0 = (int)threadIdx.x - shift; y0 < n; y0 += UN * kWThreads) {
+    V v[UN];
+#pragma unroll
+    for (int m = 0; m < UN; ++m) {
+      const int y = y0 + m * kWThreads;
+      if (y >= 0 && y < n) {
+        const int r = y / kv;
+        v[m] = UP ? span[y] : __ldcg(rows + (long long)r * pitch + (y - r * kv));
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < UN; ++m) {
+      const int y = y0 + m * kWThreads;
+      if (y >= 0 && y < n) {
+        const int r = y / kv;
+        if (UP)
+          rows[(long long)r * pitch + (y - r * kv)] = v[m];
+        else
+          span[y] = v[m];
+      }
+    }
+  }
+}
+
+// One transfer CTA: items (slab, block of planes, field) from its queue.
+template <int TJ>
+__device__ void transfer(const WaveArgs& a, int ub0, int* s_item) {
+  const WaveXfer& x = a.x;
+  const bool up = (int)blockIdx.x < a.T * a.S + x.n_up;
+  // (downloads by the tiles of the two last levels, which the skew may move)
+  const int slabs = up ? (a.g.ys + TJ - 1) / TJ : a.Q / a.ntk, fields = up ? 3 : 2;
+  const int blocks = (a.g.xs + x.planes - 1) / x.planes, per = blocks * fields;
+  while (true) {
+    if (threadIdx.x == 0) {
+      int it = atomicAdd(a.heads + (up ? 0 : 1), 1);
+      if (it >= slabs * per) it = -1;
+      if (it >= 0 && !up) {
+        // v is the level before the last, u the last
+        const int slab = it / per, f = it % fields;
+        const int* word = a.prog + ((size_t)(a.steps - 2 + f) * a.Q + slab * a.ntk) * kWPad;
+        const int j0 = slab * TJ - a.skew * ((a.steps - 2 + f) % a.T);
+        const int cols = j0 < a.g.ys && j0 + TJ > 0 ? a.ntk : 0;
+        const Patience pat(a);
+        for (int q = 0; q < cols && it >= 0; ++q)
+          for (uint32_t n = 1; w_ld_relaxed(word + (size_t)q * kWPad) < a.g.xs; ++n) {
+            __nanosleep(200);
+            if ((n & 255u) == 0 && pat.over()) {
+              give_up(a, kDevTimeoutDep);
+              it = -1;
+              break;
+            }
+          }
+        w_acquire_fence();
+      }
+      *s_item = it;
+    }
+    __syncthreads();
+    const int it = *s_item;
+    if (it < 0) return;
+    const int slab = it / per, rest = it - slab * per;
+    const int f = rest % fields, pb = rest / fields;
+    int ia = pb * x.planes, ib = min(ia + x.planes, a.g.xs);
+    int ja = slab * TJ, jb = min(ja + TJ, a.g.ys);
+    if (!up) {
+      const int j0 = ja - a.skew * ((a.steps - 2 + f) % a.T);
+      ja = max(j0, 0);
+      jb = min(j0 + TJ, a.g.ys);
+      if (jb <= ja) {
+        __syncthreads();
+        continue;
+      }
+    }
+    if (up) {
+      // the halo planes and rows come with the outermost items
+      if (pb == 0) ia -= x.hx;
+      if (ib == a.g.xs) ib += x.hx;
+      if (slab == 0) ja -= x.hy;
+      if (slab == slabs - 1) jb += x.hy;
+    }
+    // uploads: u, v, s; downloads: v (f = 0), u (f = 1) of the end
+    const int ue = ub0 ^ (a.steps & 1);
+    float* dev = up ? (f == 2 ? x.s : a.buf[f == 0 ? ub0 : ub0 ^ 1]) : a.buf[f == 1 ? ue : ue ^ 1];
+    float* host = up ? const_cast<float*>(x.hin[f]) : x.hout[f];
+    for (int i = ia; i < ib; ++i) {
+      if (up) {
+        if (x.vec) copy_rows<4, true>(a, dev, host, i, ja, jb);
+        else copy_rows<1, true>(a, dev, host, i, ja, jb);
+      } else {
+        if (x.vec) copy_rows<4, false>(a, dev, host, i, ja, jb);
+        else copy_rows<1, false>(a, dev, host, i, ja, jb);
+      }
+    }
+    __syncthreads();
+    if (up && threadIdx.x == 0) {
+      w_proxy_fence();
+      w_red_release(a.up_cnt + (size_t)slab * kWPad, 1);
+    }
+  }
+}
+
+template <int P, bool NARROW, bool STREAM>
 __global__ void __launch_bounds__(kWThreads, 1)
     k_wave(const __grid_constant__ CUtensorMap um0, const __grid_constant__ CUtensorMap um1,
            const __grid_constant__ CUtensorMap vm0, const __grid_constant__ CUtensorMap vm1,
@@ -187,6 +329,10 @@ __global__ void __launch_bounds__(kWThreads, 1)
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x / a.S, s = blockIdx.x - t * a.S;
   const int ub0 = a.ub_dev ? a.ub0 ^ __ldg(a.ub_dev) : a.ub0;
+  if (STREAM && (int)blockIdx.x >= a.T * a.S) {
+    transfer<TJ>(a, ub0, stored);
+    return;
+  }
   if (threadIdx.x < NW + 1) stored[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -212,10 +358,9 @@ __global__ void __launch_bounds__(kWThreads, 1)
     int seen = 0;
     bool ok = true;
     Turn u;
-    for (int r = 0; ok && turn(a, t, s, r, &u); ++r) {
+    for (int r = 0; ok && turn<TJ>(a, t, s, r, &u); ++r) {
       if (!u.live) continue;
-      const int jt = u.q / a.ntk, kt = u.q - jt * a.ntk;
-      const int k0 = kt * TK, j0 = jt * TJ;
+      const int k0 = u.kt * TK, j0 = u.j0;
       const int ub = ub0 ^ (u.step & 1);
       const CUtensorMap* um = ub ? &um1 : &um0;
       const CUtensorMap* vm = ub ? &vm0 : &vm1;
@@ -227,8 +372,9 @@ __global__ void __launch_bounds__(kWThreads, 1)
           break;
         }
         const int p = n - R;  // u plane of this stage
-        const int need = done + min(max(p + 1, 0), g.xs);
-        if (p >= 0 && seen < need) {
+        // (a streamed call's halo planes come with the column's slabs)
+        const int need = done + min(max(p + 1, STREAM ? 1 : 0), g.xs);
+        if (seen < need) {
           seen = w_lds_acquire(avail);
           if (seen < need) {
             const Patience pat(a);
@@ -264,7 +410,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
     // ---------------- publisher ----------------
     int done = 0;
     Turn u;
-    for (int r = 0; turn(a, t, s, r, &u); ++r) {
+    for (int r = 0; turn<TJ>(a, t, s, r, &u); ++r) {
       if (!u.live) continue;
       int* word = a.prog + ((size_t)u.step * a.Q + u.q) * kWPad;
       int out = 0;  // planes published
@@ -295,23 +441,51 @@ __global__ void __launch_bounds__(kWThreads, 1)
 
   if (warp == NW + 2) {
     // ---------------- watcher ----------------
-    // lanes 0..4: the step before, of the column and of its neighbours along
-    // k and along j; lanes 6..9: level 0, the neighbours at work in the same
+    // lanes 0..8: the step before, of the tiles (up to three) that hold the
+    // column's rows with R either side, and of those beside it along k that
+    // hold its rows; lanes 16..19: level 0, the neighbours at work in the same
     // turn, which this column may be `couple` planes ahead of
-    const int l = lane % 5;
-    const bool before = lane < 5;
+    const bool before = lane < 9;
+    const int l = before ? lane % 3 : (lane & 3) + 1;
+    const int lt = t > 0 ? t - 1 : a.T - 1;      // level of the step before
+    const int off = a.skew * lt;                 // row j lies in its tile (j + off) / TJ
     int done = 0;
     Turn u;
-    for (int r = 0; turn(a, t, s, r, &u); ++r) {
+    for (int r = 0; turn<TJ>(a, t, s, r, &u); ++r) {
       if (!u.live) continue;
-      const int jt = u.q / a.ntk, kt = u.q - jt * a.ntk;
-      const int dq = l == 1 ? -1 : l == 2 ? 1 : l == 3 ? -a.ntk : l == 4 ? a.ntk : 0;
-      bool look = before ? u.step > 0 : (lane < 10 && t == 0 && l > 0 && s + dq >= 0 && s + dq < a.S);
-      if ((l == 1 && kt == 0) || (l == 2 && kt == a.ntk - 1) || u.q + dq < 0 || u.q + dq >= a.Q) look = false;
+      const int jt = u.jt;
+      int col = u.q;
+      bool look = false;
+      if (before) {
+        const int kt = u.kt + (l == 1 ? -1 : l == 2 ? 1 : 0), reach = l == 0 ? R : 0;
+        const int first = max(u.j0 - reach, 0), last = min(u.j0 + TJ + reach, g.ys) - 1;
+        const int tile = (first + off) / TJ + lane / 3;
+        look = u.step > 0 && kt >= 0 && kt < a.ntk && tile <= (last + off) / TJ;
+        if (look) col = tile * a.ntk + kt;
+      } else if (lane >= 16 && lane < 20 && t == 0) {
+        const int dq = l == 1 ? -1 : l == 2 ? 1 : l == 3 ? -a.ntk : a.ntk;
+        look = s + dq >= 0 && s + dq < a.S &&
+               (l == 1 ? u.kt > 0 : l == 2 ? u.kt < a.ntk - 1 : l == 3 ? jt > 0 : (jt + 1) * TJ < g.ys);
+        if (look) col = u.q + dq;
+      }
       const int ahead = before ? 0 : a.couple;
-      const int* word = a.prog + ((size_t)(before ? u.step - 1 : u.step) * a.Q + u.q + dq) * kWPad;
+      const int* word = a.prog + ((size_t)(before && look ? u.step - 1 : u.step) * a.Q + col) * kWPad;
       int ready = 0;
       const Patience pat(a);
+      if (STREAM && u.step == 0) {
+        // the column's slab and the two beside it are in
+        const int slab = jt + lane - 1;
+        const bool wait = lane < 3 && slab >= 0 && slab * TJ < g.ys;
+        const int* cnt = a.up_cnt + (size_t)(wait ? slab : jt) * kWPad;
+        const int need = 3 * ((g.xs + a.x.planes - 1) / a.x.planes);
+        for (uint32_t it = 1; !__all_sync(0xffffffffu, !wait || w_ld_relaxed(cnt) >= need); ++it) {
+          __nanosleep(200);
+          if ((it & 255u) == 0 && __any_sync(0xffffffffu, pat.over())) return;
+        }
+        w_acquire_fence();
+        w_proxy_fence();
+        __syncwarp();
+      }
       for (uint32_t it = 1; ready < g.xs; ++it) {
         const int mine = look ? w_ld_relaxed(word) + ahead : g.xs;
         const int planes = min(__reduce_min_sync(0xffffffffu, mine), g.xs);
@@ -341,13 +515,12 @@ __global__ void __launch_bounds__(kWThreads, 1)
   int done = 0;
   float4 q[QN];
   Turn u;
-  for (int r = 0; turn(a, t, s, r, &u); ++r) {
+  for (int r = 0; turn<TJ>(a, t, s, r, &u); ++r) {
     if (!u.live) continue;
-    const int jt = u.q / a.ntk, kt = u.q - jt * a.ntk;
-    const int j = jt * TJ + row;
-    const int k = kt * TK + 4 * kl;
+    const int j = u.j0 + row;
+    const int k = u.kt * TK + 4 * kl;
     const int nsteps = g.xs + 2 * R;
-    const bool row_ok = j < g.ys;
+    const bool row_ok = (unsigned)j < (unsigned)g.ys;
     const int ub = ub0 ^ (u.step & 1);
     float* vrow = a.buf[ub ^ 1] + g.org + (long long)j * g.sj + k;
     const float amp = a.amps_dev ? __ldg(a.amps_dev + (size_t)u.step * a.amp_stride) : a.amps[u.step];
@@ -444,7 +617,7 @@ size_t wave_smem() {
 
 template <int P, bool NARROW>
 int occupancy_of() {
-  auto kern = k_wave<P, NARROW>;
+  auto kern = k_wave<P, NARROW, false>;
   const size_t smem = wave_smem<P, NARROW>();
   int n = 0;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -455,16 +628,22 @@ int occupancy_of() {
   return n;
 }
 
-template <int P, bool NARROW>
-cudaError_t launch_p(const WavePlan& w, const WaveArgs& a, cudaStream_t stream) {
-  auto kern = k_wave<P, NARROW>;
+template <int P, bool NARROW, bool STREAM>
+cudaError_t launch_as(const WavePlan& w, const WaveArgs& a, cudaStream_t stream) {
+  auto kern = k_wave<P, NARROW, STREAM>;
   const size_t smem = wave_smem<P, NARROW>();
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const WaveShape& sh = w.shape[NARROW ? 1 : 0];
   void* args[] = {(void*)&sh.umap[0], (void*)&sh.umap[1], (void*)&sh.vmap[0],
                   (void*)&sh.vmap[1], (void*)&sh.vmap[2], (void*)&a};
-  return cudaLaunchCooperativeKernel((const void*)kern, dim3(a.T * a.S), dim3(kWThreads), args, smem, stream);
+  const int ctas = a.T * a.S + (STREAM ? a.x.n_up + a.x.n_down : 0);
+  return cudaLaunchCooperativeKernel((const void*)kern, dim3(ctas), dim3(kWThreads), args, smem, stream);
+}
+
+template <int P, bool NARROW>
+cudaError_t launch_p(const WavePlan& w, const WaveArgs& a, cudaStream_t stream) {
+  return a.x.n_up > 0 ? launch_as<P, NARROW, true>(w, a, stream) : launch_as<P, NARROW, false>(w, a, stream);
 }
 
 }  // namespace
@@ -481,11 +660,12 @@ int wave_blocks_per_sm(int points, bool narrow) {
   }
 }
 
-size_t wave_words(int steps, int columns) { return ((size_t)steps * columns + 1) * kWPad; }
+// abort word, progress, and for a streamed call its slabs' counters and queues
+size_t wave_words(int steps, int columns) { return ((size_t)steps * columns + columns + 3) * kWPad; }
 
 cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coefs<float>& cf,
                         float* const* fld, int steps, const Source& src, const StepFeed& feed,
-                        uint32_t* dev_status, cudaStream_t stream) {
+                        uint32_t* dev_status, cudaStream_t stream, const WaveXfer* xfer) {
   if (steps < 1 || steps > w.max_steps || w.T < 1 || w.S < 1) return cudaErrorInvalidValue;
   WaveArgs a;
   a.g = g;
@@ -500,8 +680,9 @@ cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coef
   a.steps = steps;
   a.T = w.T;
   a.S = w.S;
-  a.Q = w.shape[w.narrow].Q;
+  a.Q = w.Q;
   a.shift = w.shift;
+  a.skew = w.skew;
   a.ntk = w.shape[w.narrow].ntk;
   a.couple = w.couple;
   a.abort_word = w.words;
@@ -511,6 +692,9 @@ cudaError_t launch_wave(const WavePlan& w, int points, const Geom& g, const Coef
   a.src_k = src.k;
   a.limit_ns = w.limit_ns;
   a.status = dev_status;
+  a.x = xfer ? *xfer : WaveXfer();
+  a.up_cnt = a.prog + (size_t)steps * a.Q * kWPad;
+  a.heads = a.up_cnt + (size_t)a.Q * kWPad;
   cudaError_t e = cudaMemsetAsync(w.words, 0, wave_words(steps, a.Q) * sizeof(int), stream);
   if (e != cudaSuccess) return e;
   switch (points) {

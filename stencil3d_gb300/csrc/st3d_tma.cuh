@@ -104,9 +104,9 @@ struct TbPlan {
 
 // Plan of the multi-step wave kernel (st3d_kernels_wave.cu).  The two tile
 // shapes with their maps and columns, and the progress words, belong to the
-// context; shape, T, S, shift and couple are set for each launch.
+// context; the rest is set for each launch.
 struct WaveShape {
-  int ntk = 0, Q = 0;        // tiles along k, columns
+  int tj = 0, ntj = 0, ntk = 0;  // rows of a tile, tiles along j and k
   CUtensorMap umap[2];       // halo box over the u/v pair
   CUtensorMap vmap[3];       // interior box over the pair and s
 };
@@ -114,9 +114,12 @@ struct WavePlan {
   WaveShape shape[2];        // 16 x 128 and 32 x 64 tiles
   int ctas = 0;              // CTAs the GPU holds at once
   int max_steps = 0;         // steps the words are enough for
+  int max_columns = 0;       // and columns
   int narrow = 0;            // the shape taken
   int T = 1, S = 1;          // levels, columns at work in each
+  int Q = 0;                 // columns: the tiles of all levels' rows
   int shift = 0;             // columns a level starts behind the one before
+  int skew = 0;              // rows a tile lies lower at each level
   int couple = 0;            // planes a column of level 0 may be ahead of its neighbours
   int* words = nullptr;      // progress words (device)
   size_t words_n = 0;
