@@ -122,13 +122,15 @@ typedef struct st3d_grid_desc {
  * scatter/gather kernel over the caller's array).
  * STRIDED: a 3-D strided copy, used when the host k halo exceeds the device
  * row pad.  STREAMED (st3d_iterate_host only): the DIRECT path with the
- * transfers and the steps overlapped in one launch -- CTAs copying planes of
- * u, v and s in while the others step the planes already in, as a wavefront
- * over chunks of `ichunk` planes along i (16 when 0), and copying the final
- * planes out as they are done; the same bits as the phase-by-phase call.
- * AUTO takes it for FP32 contexts on the TMA kernel's default tiles without
- * temporal blocking when v, s and u are pinned (asking for STREAMED where it
- * does not apply runs DIRECT). */
+ * transfers and the steps overlapped in one launch -- CTAs copying u, v and s
+ * in while the others step what is already in (mode W, 4 to 32 steps: rows of
+ * tiles, a pipeline of as many levels as steps; otherwise a wavefront over
+ * chunks of `ichunk` planes along i, 16 when 0), and copying the result out
+ * as it is done; the same bits as the phase-by-phase call.  AUTO takes it for
+ * FP32 contexts on the TMA kernel's default tiles without temporal blocking
+ * when v, s and u are pinned, except for mode W calls of more than 32 steps,
+ * which run faster phase by phase (asking for STREAMED where it does not apply
+ * runs DIRECT). */
 typedef enum st3d_host_path {
   ST3D_HOST_AUTO = 0,
   ST3D_HOST_STAGED = 1,

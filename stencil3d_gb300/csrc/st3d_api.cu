@@ -1047,16 +1047,16 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
 namespace {
 
 // The streamed drop-in call of the wave form as one launch of the multi-step
-// kernel with its transfer CTAs: device views of the pinned host arrays.  Takes
-// as many levels as steps where the CTAs allow, so that columns reach their last
-// step in the order they came in (25 points 512^3, 20 steps in 20 / 10 / 7
+// kernel with its transfer CTAs: device views of the pinned host arrays.  It takes
+// as many levels as steps, so that columns reach their last step in the order they
+// came in (25 points 512^3, 20 steps in 20 / 10 / 7
 // levels: 12.9 / 15.6 / 17.9 ms; chunks of planes, st3d_stream.cu, 15.9).
 // *done = false where another way is the only one.
 int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32_t iterations, bool* done) {
   const int n = (int)std::min<uint32_t>(iterations, 1u << 20), R = c->R, xs = (int)c->L.xs;
   const st3d_grid_desc& gd = c->grid;
   WavePlan w = *c->wave;
-  if (n < 4 || n > w.max_steps || w.ctas < 64) return ST3D_OK;
+  if (n < 4 || n > std::min(w.max_steps, kWaveLevels) || w.ctas < 64) return ST3D_OK;
   WaveXfer x;
   // 25 points 512^3, 20 steps, with 12 / 16 / 20 / 24 upload and 12 download
   // CTAs: 13.8 / 12.9 / 12.3 / 12.6 ms a call
@@ -1065,16 +1065,15 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
   x.planes = 16;
   const int ctas = w.ctas - x.n_up - x.n_down;
   double best = 1e300;
-  for (int nar = 0; nar < 2; ++nar)
-    for (int T = 2; T <= std::min({n, ctas, kWaveLevels}); ++T) {
-      WavePlan v = w;
-      if (!wave_layout(&v, nar, T, ctas, c->L, R)) break;
-      const double us = wave_turns(v, n) * (xs + 2 * R) * (nar ? 1.05 : 1.0) * (n > T ? 1.3 : 1.0);
-      if (us < best) {
-        best = us;
-        w = v;
-      }
+  for (int nar = 0; nar < 2; ++nar) {
+    WavePlan v = w;
+    if (!wave_layout(&v, nar, n, ctas, c->L, R)) continue;
+    const double us = wave_turns(v, n) * (xs + 2 * R) * (nar ? 1.05 : 1.0);
+    if (us < best) {
+      best = us;
+      w = v;
     }
+  }
   if (best > 1e299) return ST3D_OK;
   w.couple = kWaveCouple;
   x.R = ref_geom(gd);
@@ -1140,6 +1139,12 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   const float* hs = static_cast<const float*>(direct_view(s, hbytes));
   const float* hu = static_cast<const float*>(direct_view(u, hbytes));
   if (!hv || !hs || !hu) return ST3D_OK;
+  // many wave steps run better between the transfers than beside them (L2 or
+  // shared memory for all CTAs): 7 points 512^3, 200 steps 72 ms streamed, 60
+  // phase by phase; 64^3, 100 steps 0.98 and 0.32
+  if (c->opts.mode == ST3D_MODE_WAVE && iterations > (uint32_t)kWaveLevels &&
+      (c->wave || c->brick.nbi > 0))
+    return ST3D_OK;
   if (c->wave) {
     const int rc = iterate_host_wave(c, const_cast<float*>(hv), hs, const_cast<float*>(hu), iterations, done);
     if (rc != ST3D_OK || *done) return rc;
