@@ -176,7 +176,8 @@ typedef struct st3d_info {
   int32_t radius;             /* stencil radius */
   double bytes_per_point;     /* algorithmic HBM bytes per point per step */
   double flops_per_point;     /* reference FLOPS_PER_STENCIL (config.h:67-91) */
-  int32_t tile_j, tile_k, ichunk, temporal_block;
+  int32_t tile_j, tile_k, ichunk, temporal_block; /* st3d_plan: the kernel's base tile; the tensor-core
+                                 kernel's contexts take 16 x 152 or 32 x 64, whichever fits the grid */
   int32_t host_path;          /* st3d_host_path of the last upload or download */
   int32_t tb_tile_j;          /* rows of a temporally blocked pass's level-1 tile; 0 = none */
   int32_t device;             /* CUDA device ordinal of the context (st3d_plan: opts.device) */

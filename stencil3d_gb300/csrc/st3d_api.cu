@@ -493,7 +493,7 @@ int* Ed_lvl(st3d_ctx* c, uint64_t lvl) { return c->E + (size_t)(2 + (lvl & 1)) *
 uint32_t* Md_lvl(st3d_ctx* c, uint64_t lvl) { return c->M + (size_t)(2 + (lvl & 1)) * c->grid.xs; }
 
 int encode_map_t(CUtensorMap* m, CUtensorMapDataType dt, int eb, void* base, const Layout& L,
-                 uint32_t box_k, uint32_t box_j, uint32_t kext, uint32_t jext) {
+                 uint32_t box_k, uint32_t box_j, uint32_t kext, uint32_t jext, bool swizzle = false) {
   auto enc = get_encode();
   if (!enc) return fail(ST3D_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   cuuint64_t dims[3] = {(cuuint64_t)L.pk + L.zs + kext, (cuuint64_t)L.pj + L.ys + jext, L.ni};
@@ -501,7 +501,8 @@ int encode_map_t(CUtensorMap* m, CUtensorMapDataType dt, int eb, void* base, con
   cuuint32_t box[3] = {box_k, box_j, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(m, dt, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ST3D_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   return ST3D_OK;
@@ -614,26 +615,63 @@ bool mma_chosen(const st3d_opts& o) {
   return o.kernel == ST3D_KERNEL_AUTO && o.tile_j == 0 && o.stages == 0;
 }
 
-// Tensor-core delta-form plan (st3d_kernels_mma16.cu): 16-row x 152-column
-// tiles; tensor maps with a u box of 168 x 24 words (columns k0-8 .., rows
-// j0-R ..), d / s / lo boxes of 152 x 16 words, and interior boxes of 152 x
-// 16 over the u buffers for the stores of u^{n+1}; 8 pipeline stages (4 for
-// the pair form).
+// One step of a tile's plane takes this long (microseconds, all CTAs busy;
+// measured at 1024^3 and 512^3): the TALL tile's 16 warps are four a scheduler
+// (the WIDE tile's 19 five on three of them), and its store warp takes the
+// output copies off the thread that issues the loads, which bounds the WIDE
+// tile at 7 and 13 points and with the pair form's four stages.
+double mma_step_us(bool tall, int points, bool pair) {
+  if (points == 25) return pair ? (tall ? 0.68 : 0.84) : (tall ? 0.60 : 0.67);
+  if (pair) return tall ? 0.75 : 0.80;  // 512^3 takes 0.62 at 13 points, 1024^3 0.80 (HBM)
+  return points == 13 ? (tall ? 0.535 : 0.60) : (tall ? 0.498 : 0.575);
+}
+
+// Tensor-core delta-form plan (st3d_kernels_mma16.cu): the tile (MmaTile,
+// st3d_tma.cuh) with the shorter estimated step, which weighs how well it
+// fills the rows (multiples of 152 or 64 columns, 16 or 32 rows) against the
+// time above; WIDE where the request names a tile height or depth.  Measured,
+// us a step WIDE and TALL: FP16 25 points 512^3 326 / 290 (492 tile steps either
+// way; 1024^3, 3096 against 3672, stays WIDE: 2085), 7 points 512^3 272 / 234,
+// 1024^3 1785 / 1720; F16_HL 25 points 512^3 396 / 324, 1024^3 2686 / 2425, 13
+// points 512^3 388 / 306; the worst met, F16_HL 7 points 200 x 700 x 500, 205 / 208.
 int plan_mma16(st3d_ctx* c, int sm_count, int max_smem) {
   Tma16Plan* p = new (std::nothrow) Tma16Plan();
   if (!p) return fail(ST3D_ERR_NOMEM, "host allocation failed");
   const int R = c->R;
   p->radius = R;
-  p->tj = 16;
   p->delta = true;
   p->pair = c->pair;
   p->mma = true;
   p->nb = 1;
-  p->nv = c->pair ? 4 : 8;
-  p->smem = mma16_smem_bytes(p->nv, R, c->pair);
-  const int per_sm =
-      (int)p->smem <= max_smem ? mma16_blocks_per_sm(c->opts.storage, c->opts.points, *p) : 0;
-  if (per_sm < 1) {
+  const bool named = c->opts.tile_j > 0 || c->opts.stages > 0;
+  double best = 1e300;
+  for (int tall = 0; tall < (named ? 1 : 2); ++tall) {
+    Tma16Plan q = *p;
+    q.tall = tall != 0;
+    q.tj = tall ? MmaTile<true>::TJ : MmaTile<false>::TJ;
+    q.tk = tall ? MmaTile<true>::TK : MmaTile<false>::TK;
+    q.threads = tall ? MmaTile<true>::THREADS : MmaTile<false>::THREADS;
+    q.nv = c->pair ? (tall ? kMmaStages<true, true> : kMmaStages<false, true>)
+                   : (tall ? kMmaStages<true, false> : kMmaStages<false, false>);
+    q.smem = mma16_smem_bytes(q.nv, c->pair, q.tall);
+    const int per_sm =
+        (int)q.smem <= max_smem ? mma16_blocks_per_sm(c->opts.storage, c->opts.points, q) : 0;
+    if (per_sm < 1) continue;
+    q.ntj = (int)((c->L.ys + q.tj - 1) / q.tj);
+    q.ntk = (int)((c->L.zs + q.tk - 1) / q.tk);
+    const int ctas = sm_count * per_sm;
+    q.ichunk = c->opts.ichunk > 0 ? c->opts.ichunk : tma_pick_ichunk((int)c->L.xs, q.ntj * q.ntk, ctas, R);
+    q.nti = (int)((c->L.xs + q.ichunk - 1) / q.ichunk);
+    q.units = q.ntj * q.ntk * q.nti;
+    q.grid = ctas < q.units ? ctas : q.units;
+    const double us = (double)((q.units + ctas - 1) / ctas) * (std::min(q.ichunk, (int)c->L.xs) + 2 * R) *
+                      mma_step_us(q.tall, c->opts.points, c->pair);
+    if (us < best) {
+      best = us;
+      *p = q;
+    }
+  }
+  if (best > 1e299) {
     delete p;
     return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel does not fit in shared memory");
   }
@@ -643,28 +681,24 @@ int plan_mma16(st3d_ctx* c, int sm_count, int max_smem) {
     return fail(ST3D_ERR_NOMEM, "cudaMalloc of the plane records failed");
   }
   c->bytes += (size_t)c->L.xs * sizeof(MmaRecord);
-  p->ntj = (int)((c->L.ys + 15) / 16);
-  p->ntk = (int)((c->L.zs + kMmaTK - 1) / kMmaTK);
-  const int ctas = sm_count * per_sm;
-  p->ichunk = c->opts.ichunk > 0 ? c->opts.ichunk : tma_pick_ichunk((int)c->L.xs, p->ntj * p->ntk, ctas, R);
-  p->nti = (int)((c->L.xs + p->ichunk - 1) / p->ichunk);
-  p->units = p->ntj * p->ntk * p->nti;
-  p->grid = ctas < p->units ? ctas : p->units;
-  p->threads = (kMmaTK / 8 + 1) * 32;
   const CUtensorMapDataType w16 =
       c->opts.storage == ST3D_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const uint32_t uw = p->tall ? MmaTile<true>::UW : MmaTile<false>::UW;
   int ok = ST3D_OK;
+  // d, s, lo and the interior box of u^{n+1}: tk x tj words, swizzled for TALL
+  auto tile_map = [&](CUtensorMap* m, CUtensorMapDataType dt, void* base) {
+    return encode_map_t(m, dt, 2, base, c->L, p->tk, p->tj, 0, 0, p->tall);
+  };
   for (int f = 0; f < 2 && ok == ST3D_OK; ++f) {
-    ok = encode_map_t(&p->uhi[f], w16, 2, c->fld[f], c->L, kMmaTK + 16, 24, 8, c->L.pj);
-    // the interior box the kernel stores u^{n+1} through
-    if (ok == ST3D_OK) ok = encode_map_t(&p->vhi[f], w16, 2, c->fld[f], c->L, kMmaTK, 16, 0, 0);
+    ok = encode_map_t(&p->uhi[f], w16, 2, c->fld[f], c->L, uw, p->tj + 8, 8, c->L.pj);
+    if (ok == ST3D_OK) ok = tile_map(&p->vhi[f], w16, c->fld[f]);
     if (ok == ST3D_OK && c->pair)
-      ok = encode_map_t(&p->lo[f], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, c->lo[f], c->L, kMmaTK, 16, 0, 0);
+      ok = tile_map(&p->lo[f], CU_TENSOR_MAP_DATA_TYPE_UINT16, c->lo[f]);
     else if (ok == ST3D_OK)
       p->lo[f] = p->uhi[f];  // unused without the pair form
   }
-  if (ok == ST3D_OK) ok = encode_map_t(&p->vhi[2], w16, 2, c->fld[2], c->L, kMmaTK, 16, 0, 0);
-  if (ok == ST3D_OK) ok = encode_map_t(&p->dmap, w16, 2, c->fld[3], c->L, kMmaTK, 16, 0, 0);
+  if (ok == ST3D_OK) ok = tile_map(&p->vhi[2], w16, c->fld[2]);
+  if (ok == ST3D_OK) ok = tile_map(&p->dmap, w16, c->fld[3]);
   if (ok != ST3D_OK) {
     cudaFree(p->mma_rec);
     delete p;
@@ -1798,7 +1832,7 @@ int st3d_get_info(const st3d_ctx* c, st3d_info* info) {
   info->bytes_per_point = c->tb ? 20.0 / c->tb->T : f16_bytes(c->opts.storage, c->opts.points, c->eb);
   info->flops_per_point = c->opts.points == 2 ? 2 : c->opts.points == 7 ? 12 : c->opts.points == 13 ? 29 : 41;
   info->tile_j = c->tma ? c->tma->tj : c->tma16 ? c->tma16->tj : 0;
-  info->tile_k = (c->tma16 && c->tma16->mma) ? kMmaTK : (c->tma || c->tma16) ? kTmaTK : 0;
+  info->tile_k = c->tma16 ? c->tma16->tk : c->tma ? kTmaTK : 0;
   info->ichunk = c->tma ? c->tma->ichunk : c->tma16 ? c->tma16->ichunk : c->ichunk;
   info->temporal_block = c->opts.temporal_block;
   info->host_path = c->host_path;

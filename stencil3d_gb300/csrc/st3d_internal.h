@@ -300,7 +300,7 @@ cudaError_t launch_scales_delta(const Geom& g, int R, const Delta16Step& st, flo
                                 cudaStream_t stream);
 // The delta form with the j and k neighbour sums on the tensor cores
 // (st3d_kernels_mma16.cu); plan fields mma / nb.
-size_t mma16_smem_bytes(int nv, int R, bool pair);
+size_t mma16_smem_bytes(int nv, bool pair, bool tall);
 int mma16_blocks_per_sm(int storage, int points, const Tma16Plan& pl);
 cudaError_t launch_mma16(int storage, int points, const Tma16Plan& pl, const Geom& g,
                          const Coefs<float>& cf, const Delta16Step& st, const Source& src,

@@ -42,26 +42,37 @@
 // FP16 powers of two end at 2^-24 = 2^(39-15) below 2^X): its contribution
 // is far below FP32 rounding of the sum.
 //
-// Structure (one CTA per SM, persistent over 16-row x 152-column x
-// ichunk-plane units): a producer thread streams, per step, the u plane i+R
-// (rows j0-R .. j0-R+23, columns k0-8 .. k0+159) and, for the centre plane
-// i, d, s (the lo words of u) over columns k0 .. k0+151 and the plane's
-// record, through an mbarrier ring of 8 stages (4 for the pair form); 19
-// consumer warps each own one 16x8 block (20 warps with the producer: five
-// on some schedulers, within the 96 registers a thread that leaves; the
-// kernel takes 81-87).  The row pitches (336 and 304 bytes) put the eight
-// rows of every ldmatrix in distinct banks.  Each warp writes its block of
-// u^{n+1}, d^{n+1} (and the lo words) into the stage's s, d (and lo) slots, whose
-// inputs it has read, with zero words at the points outside the grid; once
-// every warp has released the stage the producer stores the three tiles with
-// TMA (whole lines, clipped by the tensor maps' extents) and waits for the
-// stores to read shared memory before it loads the slots again.  A store
-// whose clipped row ends inside a 16-byte segment was seen to write the rest
-// of that segment (the zero halo along k when zs is not a multiple of 8), so
-// the outputs outside the grid are zeros, the value the halo holds.  Waits
-// are bounded; after a timeout the consumers keep stepping and arriving
-// without waiting, so that the producer's bounded drain ends and every CTA
-// returns (the status word marks the results void).
+// Structure (one CTA per SM, persistent over tile x ichunk-plane units; the
+// tile is WIDE, 16 rows x 152 columns, or TALL, 32 x 64): a load thread
+// streams, per step, the u plane i+R (rows j0-R .. j0+TJ+7-R, columns k0-8 ..)
+// and, for the centre plane i, d, s (the lo words of u) and the plane's record,
+// through an mbarrier ring of 8 stages (4 for the pair form's WIDE tiles);
+// 19 or 16 consumer warps each own one 16x8 block.  Each warp writes its block
+// of u^{n+1}, d^{n+1} (and the lo words) into the stage's s, d (and lo) slots,
+// whose inputs it has read, with zero words at the points outside the grid;
+// once every warp has released the stage the three tiles are stored with TMA
+// (whole lines, clipped by the tensor maps' extents), and the slots are loaded
+// again when the stores have read them.  A store whose clipped row ends inside
+// a 16-byte segment was seen to write the rest of that segment (the zero halo
+// along k when zs is not a multiple of 8), so the outputs outside the grid are
+// zeros, the value the halo holds.  Waits are bounded; after a timeout the
+// consumers keep stepping and arriving without waiting, so that the bounded
+// drains end and every CTA returns (the status word marks the results void).
+//
+// What bounds a step is the time a warp takes through its chain of ldmatrix,
+// mma and conversions while the scheduler's other warps fill in: a step of the
+// WIDE tile takes 0.67 us at 25 points with five warps on three of the
+// schedulers (20 with the copy warp, the most that leaves 96 registers a
+// thread), one of the TALL tile 0.59 us with four on each.  WIDE does more a
+// step; TALL fits grids in smaller units (512 = 8 x 64 against 3.4 x 152) and
+// has room for a store warp of its own: with one thread for loads and stores a
+// step never took less than 0.55 us, a 7-point step now takes 0.50, and the
+// pair form, whose smaller slots take 8 stages, 0.66 for 0.80.  plan_mma16
+// (st3d_api.cu) chooses.  Shared memory: the row pitches of the u boxes (336 and
+// 176 bytes) and of the WIDE d / s / lo tiles (304) put the eight rows of every
+// ldmatrix in distinct banks; the 128-byte rows of the TALL ones do by the copy
+// engine's swizzle.  Two blocks a warp (8 warps of 32 x 64, 12 of 48 x 64) were
+// slower, 0.70 and 0.94 us: fewer warps hide less.
 #include <math.h>
 #include <string.h>
 
@@ -74,15 +85,7 @@ namespace st3d {
 
 namespace {
 
-constexpr int kMTJ = 16;         // rows per tile (one 16-row mma block)
-constexpr int kMTK = kMmaTK;     // columns per tile (nineteen 8-column blocks)
-constexpr int kMCW = kMmaTK / 8; // consumer warps, one 8-column block each
-constexpr int kMUW = kMTK + 16;  // u tile row: k0-8 .. k0+159, 336 bytes
-constexpr int kMVW = kMTK;       // d / s / lo tile row: k0 .. k0+151, 304 bytes
-constexpr int kMUH = kMTJ + 8;   // u tile rows: j0-R .. j0-R+23
-constexpr int kMNV = 8;          // pipeline stages (4 for the pair form, whose third tile per stage
-                                 // would not fit 8)
-constexpr int kMNU = 16;         // u ring slots (>= NV + 2R; a power of two)
+constexpr int kMNU = 16;         // u ring slots (>= stages + 2R; a power of two)
 
 template <int P>
 struct RadM {
@@ -249,33 +252,38 @@ __device__ __forceinline__ float amax4m(const P4& x, uint32_t v) {
   return m;
 }
 
-template <int KIND, int P, bool PAIR>
-__global__ void __launch_bounds__((kMCW + 1) * 32, 1)
+template <int KIND, int P, bool PAIR, bool TALL>
+__global__ void __launch_bounds__(MmaTile<TALL>::THREADS, 1)
     k_mma16(const __grid_constant__ CUtensorMap umap, const __grid_constant__ CUtensorMap dmap,
             const __grid_constant__ CUtensorMap smap, const __grid_constant__ CUtensorMap lmap,
             const __grid_constant__ CUtensorMap uomap, const __grid_constant__ CUtensorMap lomap,
             const Mma16Args a) {
   constexpr int R = RadM<P>::value;
-  constexpr int NV = PAIR ? kMNV / 2 : kMNV;
+  using Tile = MmaTile<TALL>;
+  constexpr int NV = kMmaStages<TALL, PAIR>;
   constexpr int NU = kMNU;
-  constexpr int CW = kMCW;
-  constexpr uint32_t UBYTES = kMUW * kMUH * 2;
-  constexpr uint32_t VBYTES = kMVW * kMTJ * 2;
+  constexpr int CW = Tile::CW;
+  constexpr int TJ = Tile::TJ, TK = Tile::TK, UW = Tile::UW;
+  constexpr int VP = TK * 2;  // bytes a d / s / lo row
+  constexpr uint32_t UBYTES = UW * Tile::UH * 2;
+  constexpr uint32_t VBYTES = VP * TJ;
   constexpr uint32_t RBYTES = sizeof(MmaRecord);
   constexpr int USLOT = (UBYTES + 127) / 128 * 128;
   constexpr int VSLOT = (VBYTES + 127) / 128 * 128;
   static_assert(NU >= NV + 2 * R && (NU & (NU - 1)) == 0 && (NV & (NV - 1)) == 0, "ring sizes");
   static_assert(sizeof(MmaRecord) % 128 == 0, "record size");
+  static_assert(!TALL || (VSLOT % 1024 == 0 && NU * USLOT % 1024 == 0), "swizzled tiles start on 1024 bytes");
 
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* ur = smem;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char* ur = smem;  // the u ring first: 1.5 % of a WIDE step at 25 points
   unsigned char* dr = ur + NU * USLOT;
   unsigned char* sr = dr + NV * VSLOT;
   unsigned char* lr = sr + NV * VSLOT;
   MmaRecord* rec = reinterpret_cast<MmaRecord*>(lr + (PAIR ? NV * VSLOT : 0));
   uint64_t* full = reinterpret_cast<uint64_t*>(rec + NV);
   uint64_t* empty = full + NV;
-  uint32_t* smax_u = reinterpret_cast<uint32_t*>(empty + NV);
+  uint64_t* drained = empty + NV;  // TALL: the stage's outputs have left
+  uint32_t* smax_u = reinterpret_cast<uint32_t*>(drained + NV);
   uint32_t* smax_d = smax_u + NV;
   int* splane = reinterpret_cast<int*>(smax_d + NV);
   int* sj0 = splane + NV;  // tile origin of the stage's step (its outputs' store)
@@ -290,6 +298,7 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
     for (int s = 0; s < NV; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], CW * 32);
+      mbar_init(&drained[s], 1);
       smax_u[s] = 0u;
       smax_d[s] = 0u;
       splane[s] = -1;
@@ -299,7 +308,107 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
   }
   __syncthreads();
 
-  if (warp == CW) {
+  if (TALL && warp == CW) {
+    // ---------------- loads (lane 0) -----------------
+    if (lane != 0) return;
+    tma_prefetch_desc(&umap);
+    tma_prefetch_desc(&dmap);
+    tma_prefetch_desc(&smap);
+    if (PAIR) tma_prefetch_desc(&lmap);
+    uint32_t h = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < a.units && ok; unit += gridDim.x) {
+      const int ic = unit / a.ntjk;
+      const int rem = unit - ic * a.ntjk;
+      const int jt = rem / a.ntk;
+      const int kt = rem - jt * a.ntk;
+      const int k0 = kt * TK, j0 = jt * TJ;
+      const int ia = ic * a.ichunk;
+      const int ib = min(ia + a.ichunk, g.xs);
+      const int nsteps = (ib - ia) + 2 * R;
+      for (int n = 0; n < nsteps; ++n, ++h) {
+        const int stage = (int)(h & (NV - 1));
+        if (h >= (uint32_t)NV && !mbar_wait_bounded(&drained[stage], (h / NV - 1) & 1u, a.timeout_ns)) {
+          atomicExch(a.status, (uint32_t)kDevTimeoutEmpty);
+          ok = false;
+          break;
+        }
+        const int p = ia - R + n;
+        const bool has_ds = n >= 2 * R;
+        const int i = ia + n - 2 * R;
+        mbar_arrive_expect_tx(&full[stage], UBYTES + (has_ds ? (PAIR ? 3u : 2u) * VBYTES + RBYTES : 0u));
+        tma_load_3d(ur + (h & (NU - 1)) * USLOT, &umap, &full[stage], g.pk + k0 - 8, g.pj + j0 - R,
+                    g.pi + p);
+        if (has_ds) {
+          tma_load_3d(dr + stage * VSLOT, &dmap, &full[stage], g.pk + k0, g.pj + j0, g.pi + i);
+          tma_load_3d(sr + stage * VSLOT, &smap, &full[stage], g.pk + k0, g.pj + j0, g.pi + i);
+          if (PAIR) tma_load_3d(lr + stage * VSLOT, &lmap, &full[stage], g.pk + k0, g.pj + j0, g.pi + i);
+          bulk_load(&rec[stage], &a.rec[i], RBYTES, &full[stage]);
+        }
+      }
+    }
+    // no copy in flight when this thread leaves
+    for (uint32_t m = h > (uint32_t)NV ? h - NV : 0u; m < h; ++m)
+      if (!mbar_wait_bounded(&full[m & (NV - 1)], (m / NV) & 1u, a.timeout_ns))
+        atomicExch(a.status, (uint32_t)kDevTimeoutEmpty);
+    return;
+  }
+  if (TALL && warp == CW + 1) {
+    // ---------------- stores (lane 0) -----------------
+    // A finished step's outputs sit in its stage's d, s and lo slots; they go
+    // out as tile stores, and the stage is handed back to the loads one step
+    // later, when they have read it.
+    if (lane != 0) return;
+    tma_prefetch_desc(&uomap);
+    if (PAIR) tma_prefetch_desc(&lomap);
+    uint32_t h = 0;
+    int pending = -1;  // stage whose stores are still reading
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < a.units && ok; unit += gridDim.x) {
+      const int ic = unit / a.ntjk;
+      const int rem = unit - ic * a.ntjk;
+      const int jt = rem / a.ntk;
+      const int kt = rem - jt * a.ntk;
+      const int x = g.pk + kt * TK, y = g.pj + jt * TJ;
+      const int ia = ic * a.ichunk;
+      const int ib = min(ia + a.ichunk, g.xs);
+      const int nsteps = (ib - ia) + 2 * R;
+      for (int n = 0; n < nsteps; ++n, ++h) {
+        const int stage = (int)(h & (NV - 1));
+        if (!mbar_wait_bounded(&empty[stage], (h / NV) & 1u, a.timeout_ns)) {
+          atomicExch(a.status, (uint32_t)kDevTimeoutEmpty);
+          ok = false;
+          break;
+        }
+        if (n >= 2 * R) {
+          const int i = ia + n - 2 * R;
+          tma_store_3d(&uomap, sr + stage * VSLOT, x, y, g.pi + i);
+          tma_store_3d(&dmap, dr + stage * VSLOT, x, y, g.pi + i);
+          if (PAIR) tma_store_3d(&lomap, lr + stage * VSLOT, x, y, g.pi + i);
+          bulk_commit();
+          if (smax_u[stage]) atomicMax(&a.Mu_out[i], smax_u[stage]);
+          if (smax_d[stage]) atomicMax(&a.Md_out[i], smax_d[stage]);
+          smax_u[stage] = 0u;
+          smax_d[stage] = 0u;
+          if (pending >= 0) {
+            bulk_wait_read1();
+            mbar_arrive(&drained[pending]);
+          }
+          pending = stage;
+        } else {
+          if (pending >= 0) {
+            bulk_wait_read0();
+            mbar_arrive(&drained[pending]);
+            pending = -1;
+          }
+          mbar_arrive(&drained[stage]);
+        }
+      }
+    }
+    bulk_wait_all();
+    return;
+  }
+  if (!TALL && warp == CW) {
     // ---------------- producer (lane 0 drives the pipeline) -----------------
     if (lane != 0) return;
     // The outputs of a finished step sit in its stage's d (d^{n+1}), s
@@ -347,7 +456,7 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
       const int rem = unit - ic * a.ntjk;
       const int jt = rem / a.ntk;
       const int kt = rem - jt * a.ntk;
-      const int k0 = kt * kMTK, j0 = jt * kMTJ;
+      const int k0 = kt * TK, j0 = jt * TJ;
       const int ia = ic * a.ichunk;
       const int ib = min(ia + a.ichunk, g.xs);
       const int nsteps = (ib - ia) + 2 * R;
@@ -411,7 +520,8 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
 
   // ---------------- consumers: one 16x8 block per warp ----------------
   const int g8 = lane >> 2, t4 = lane & 3;
-  const int kb = warp;  // the warp's 8-column block
+  const int kb = TALL ? warp & 7 : warp;     // the warp's 8-column block
+  const int jb = TALL ? (warp >> 3) * 16 : 0;  // and its first row
   uint32_t wkh[3], wkl[3], wjh[6], wjl[6];
   band_fragments<KIND>(a, R, g8, t4, wkh, wkl, wjh, wjl);
   const bool need_lo = a.need_lo != 0;
@@ -427,15 +537,18 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
   //   vbase: d rows 0..15 (lanes 0..15) and s rows 0..15 (lanes 16..31);
   //   lbase: the lo words of u, rows 0..15.
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8;
-  const uint32_t u0s = smem_u32(ur);
-  const uint32_t abase = u0s + (uint32_t)(((R + lrow) * kMUW + kb * 8 + (lane >> 4) * 8) * 2);
-  const uint32_t bbase = u0s + (uint32_t)((((lane & 7) + 8 * min(lane >> 3, 2)) * kMUW + kb * 8 + 8) * 2);
-  const uint32_t pbase = u0s + (uint32_t)(((R + lrow) * kMUW + kb * 8 + 8) * 2);
-  const uint32_t vbase = smem_u32(lane < 16 ? dr : sr) + (uint32_t)((lrow * kMVW + kb * 8) * 2);
-  const uint32_t lbase = smem_u32(lr) + (uint32_t)((lrow * kMVW + kb * 8) * 2);
+  const uint32_t u0s = smem_u32(ur) + (uint32_t)(jb * UW * 2);
+  const uint32_t abase = u0s + (uint32_t)(((R + lrow) * UW + kb * 8 + (lane >> 4) * 8) * 2);
+  const uint32_t bbase = u0s + (uint32_t)((((lane & 7) + 8 * min(lane >> 3, 2)) * UW + kb * 8 + 8) * 2);
+  const uint32_t pbase = u0s + (uint32_t)(((R + lrow) * UW + kb * 8 + 8) * 2);
+  // (TALL: 128-byte rows, the 16-byte units of a row exchanged by the copy
+  // engine's 128-byte swizzle, unit ^ (row mod 8))
+  const uint32_t voff = (uint32_t)((jb + lrow) * VP + (TALL ? kb ^ (lane & 7) : kb) * 16);
+  const uint32_t vbase = smem_u32(lane < 16 ? dr : sr) + voff;
+  const uint32_t lbase = smem_u32(lr) + voff;
   const int rsign = lane < 16 ? -1 : 1;
   // this lane's output words in a d / s / lo slot: rows g and g+8, columns 8kb + 2t
-  const uint32_t obase = (uint32_t)((g8 * kMVW + kb * 8 + 2 * t4) * 2);
+  const uint32_t obase = (uint32_t)((jb + g8) * VP + (TALL ? kb ^ g8 : kb) * 16 + 4 * t4);
 
   uint32_t h = 0;
   bool failed = false;
@@ -444,15 +557,15 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
     const int rem = unit - ic * a.ntjk;
     const int jt = rem / a.ntk;
     const int kt = rem - jt * a.ntk;
-    const int j0 = jt * kMTJ, k0 = kt * kMTK;
+    const int j0 = jt * TJ, k0 = kt * TK;
     const int ia = ic * a.ichunk;
     const int ib = min(ia + a.ichunk, g.xs);
     const int nsteps = (ib - ia) + 2 * R;
     // this lane's points: rows jr0, jr0 + 8, columns kc, kc + 1
-    const int jr0 = j0 + g8;
+    const int jr0 = j0 + jb + g8;
     const int kc = k0 + 8 * kb + 2 * t4;
     const bool r0 = jr0 < g.ys, r1 = jr0 + 8 < g.ys, c0ok = kc < g.zs, c1ok = kc + 1 < g.zs;
-    const bool whole = j0 + kMTJ <= g.ys && k0 + kMTK <= g.zs;
+    const bool whole = j0 + TJ <= g.ys && k0 + TK <= g.zs;
     // points inside the grid (bit c: component c of the lane's P4) for the
     // plane maxima; the tile stores clip the rest
     const uint32_t vbits = (r0 && c0ok ? 1u : 0u) | (r0 && c1ok ? 2u : 0u) | (r1 && c0ok ? 4u : 0u) |
@@ -462,8 +575,8 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
     // k is the zero halo (and the zero row pad after it)
     const uint32_t cmask = (c0ok ? 0x0000ffffu : 0u) | (c1ok ? 0xffff0000u : 0u);
     const uint32_t om0 = r0 ? cmask : 0u, om1 = r1 ? cmask : 0u;
-    const bool src_unit = a.src.i >= ia && a.src.i < ib && a.src.j >= j0 && a.src.j < j0 + kMTJ &&
-                          a.src.k >= k0 && a.src.k < k0 + kMTK;
+    const bool src_unit = a.src.i >= ia && a.src.i < ib && a.src.j >= j0 && a.src.j < j0 + TJ &&
+                          a.src.k >= k0 && a.src.k < k0 + TK;
     for (int n = 0; n < nsteps; ++n) {
       const uint32_t hh = h + (uint32_t)n;
       const uint32_t stage = hh & (NV - 1);
@@ -559,13 +672,13 @@ __global__ void __launch_bounds__((kMCW + 1) * 32, 1)
           unsigned char* so = sr + stage * VSLOT + obase;
           unsigned char* dout = dr + stage * VSLOT + obase;
           *reinterpret_cast<uint32_t*>(so) = uwo.x & om0;
-          *reinterpret_cast<uint32_t*>(so + 8 * kMVW * 2) = uwo.y & om1;
+          *reinterpret_cast<uint32_t*>(so + 8 * VP) = uwo.y & om1;
           *reinterpret_cast<uint32_t*>(dout) = dwo.x & om0;
-          *reinterpret_cast<uint32_t*>(dout + 8 * kMVW * 2) = dwo.y & om1;
+          *reinterpret_cast<uint32_t*>(dout + 8 * VP) = dwo.y & om1;
           if (PAIR) {
             unsigned char* lo = lr + stage * VSLOT + obase;
             *reinterpret_cast<uint32_t*>(lo) = ulo.x & om0;
-            *reinterpret_cast<uint32_t*>(lo + 8 * kMVW * 2) = ulo.y & om1;
+            *reinterpret_cast<uint32_t*>(lo + 8 * VP) = ulo.y & om1;
           }
           fence_proxy_async_smem();
         }
@@ -651,17 +764,24 @@ __global__ void k_mma_records(int xs, int R, const int* __restrict__ Eu, const i
   rec[i] = o;
 }
 
-template <int KIND, int P, bool PAIR>
-cudaError_t launch_p(const Tma16Plan& pl, const Mma16Args& args, const CUtensorMap* maps,
+template <int KIND, int P, bool PAIR, bool TALL>
+cudaError_t launch_t(const Tma16Plan& pl, const Mma16Args& args, const CUtensorMap* maps,
                      cudaStream_t stream, int* occupancy_out) {
-  if (pl.nv != (PAIR ? kMNV / 2 : kMNV) || pl.nb != 1) return cudaErrorInvalidConfiguration;
-  auto kern = k_mma16<KIND, P, PAIR>;
-  const int threads = (kMCW + 1) * 32;
+  if (pl.nv != kMmaStages<TALL, PAIR> || pl.nb != 1) return cudaErrorInvalidConfiguration;
+  auto kern = k_mma16<KIND, P, PAIR, TALL>;
+  const int threads = MmaTile<TALL>::THREADS;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
   if (e != cudaSuccess) return e;
   if (occupancy_out) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy_out, kern, threads, pl.smem);
   kern<<<pl.grid, threads, pl.smem, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], args);
   return cudaGetLastError();
+}
+
+template <int KIND, int P, bool PAIR>
+cudaError_t launch_p(const Tma16Plan& pl, const Mma16Args& args, const CUtensorMap* maps,
+                     cudaStream_t stream, int* occ) {
+  return pl.tall ? launch_t<KIND, P, PAIR, true>(pl, args, maps, stream, occ)
+                 : launch_t<KIND, P, PAIR, false>(pl, args, maps, stream, occ);
 }
 
 template <int KIND, bool PAIR>
@@ -696,12 +816,15 @@ bool exact16(int storage, float w) {
 
 }  // namespace
 
-size_t mma16_smem_bytes(int nv, int R, bool pair) {
-  (void)R;
-  const size_t uslot = ((size_t)kMUW * kMUH * 2 + 127) / 128 * 128;
-  const size_t vslot = ((size_t)kMVW * kMTJ * 2 + 127) / 128 * 128;
-  return (size_t)kMNU * uslot + (pair ? 3 : 2) * (size_t)nv * vslot + (size_t)nv * sizeof(MmaRecord) +
-         2 * (size_t)nv * 8 + 5 * (size_t)nv * 4 + 128;
+size_t mma16_smem_bytes(int nv, bool pair, bool tall) {
+  auto bytes = [&](auto t) {
+    using Tile = decltype(t);
+    const size_t uslot = ((size_t)Tile::UW * Tile::UH * 2 + 127) / 128 * 128;
+    const size_t vslot = ((size_t)Tile::TK * Tile::TJ * 2 + 127) / 128 * 128;
+    return (size_t)kMNU * uslot + (pair ? 3 : 2) * (size_t)nv * vslot + (size_t)nv * sizeof(MmaRecord) +
+           3 * (size_t)nv * 8 + 5 * (size_t)nv * 4 + 128;
+  };
+  return tall ? bytes(MmaTile<true>()) : bytes(MmaTile<false>());
 }
 
 int mma16_blocks_per_sm(int storage, int points, const Tma16Plan& pl) {

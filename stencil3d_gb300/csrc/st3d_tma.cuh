@@ -18,6 +18,22 @@ constexpr int kTmaUKW = kTmaTK + 2 * kTmaKHalo; // smem row width of a u tile
 // blocks, one consumer warp each).
 constexpr int kMmaTK = 152;
 
+// The two tiles of the tensor-core kernel (st3d_kernels_mma16.cu): WIDE, 16
+// rows x 152 columns, 19 consumer warps and one copy warp; TALL, 32 x 64, 16
+// consumer warps and a load and a store warp.
+template <bool TALL>
+struct MmaTile {
+  static constexpr int TJ = TALL ? 32 : 16;
+  static constexpr int TK = TALL ? 64 : kMmaTK;
+  static constexpr int UW = TALL ? 88 : kMmaTK + 16;  // u box: columns k0-8 .. (odd 16-byte units a row)
+  static constexpr int UH = TJ + 8;                   // rows j0-R ..
+  static constexpr int CW = TJ / 16 * (TK / 8);       // consumer warps, one 16x8 block each
+  static constexpr int THREADS = (CW + (TALL ? 2 : 1)) * 32;
+};
+// pipeline stages: the pair form's third output tile leaves 4 stages of the WIDE tile
+template <bool TALL, bool PAIR>
+constexpr int kMmaStages = PAIR && !TALL ? 4 : 8;
+
 struct TmaPlan {
   int tj = 16;      // rows per tile (consumer warps)
   int nv = 3;       // pipeline stages (v/s ring depth); u ring has nv + R slots
@@ -58,8 +74,9 @@ struct Tma16Plan {
   uint64_t timeout_ns = 4000000000ull;
   bool delta = false;     // FP16 / BF16 delta form (st3d_kernels_delta16.cu)
   bool pair = false;      // F16_HL: u as an FP16 hi/lo pair; lo[] are its lo words
-  bool mma = false;       // delta form on the tensor-core kernel (st3d_kernels_mma16.cu):
-                          // 16 x kMmaTK tiles, u box (kMmaTK+16) x 24, d/s/lo boxes kMmaTK x 16
+  bool mma = false;       // delta form on the tensor-core kernel (st3d_kernels_mma16.cu)
+  bool tall = false;      // ... on its 32 x 64 tile; else 16 x 152
+  int tk = 128;           // columns per tile
   int nb = 1;             // mma kernel: 8-column blocks per consumer warp
   MmaRecord* mma_rec = nullptr;  // mma kernel: one record per i-plane (device)
   CUtensorMap uhi[2];
