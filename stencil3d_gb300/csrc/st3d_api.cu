@@ -811,27 +811,26 @@ float* stage_slot(st3d_ctx* c, int slot) {
   return reinterpret_cast<float*>(static_cast<char*>(c->stage) + (size_t)slot * host_array_bytes(c));
 }
 
-// Encode a (or a - b) from the staging slots into 16-bit words with per-plane
-// maxima M and scales E; the halo of a (and b) must be zero.
-int encode_staged16(st3d_ctx* c, const float* a, const float* b, void* words, uint32_t* M, int* E,
-                    const char* what, void* lo16 = nullptr) {
+// Encode s from `a` (the caller's device array or slot 0) into 16-bit words
+// with per-plane maxima and scales; its halo must be zero.
+int encode_s16(st3d_ctx* c, const float* a) {
   const st3d_grid_desc& g = c->grid;
   const RefGeom R = ref_geom(g);
   const int hx = g.xh < 4 ? (int)g.xh : 4, hy = g.yh < 4 ? (int)g.yh : 4, hz = (int)g.zh;
+  uint32_t* M = M_s(c);
   ST3D_CUDA(cudaMemsetAsync(M, 0, g.xs * sizeof(uint32_t), c->stream));
   ST3D_CUDA(cudaMemsetAsync(c->halo_max, 0, sizeof(uint32_t), c->stream));
-  cudaError_t e = launch_plane_max_ref(R, a, M, c->halo_max, hx, hy, hz, c->stream, b);
+  cudaError_t e = launch_plane_max_ref(R, a, M, c->halo_max, hx, hy, hz, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "plane maximum kernel");
-  e = launch_ref_to_dev16(word_storage(c->opts.storage), c->L, R, a, (uint16_t*)words, nullptr, M, E,
-                          hx, hy, hz, c->stream, b, (uint16_t*)lo16);
+  e = launch_ref_to_dev16(word_storage(c->opts.storage), c->L, R, a, (uint16_t*)c->fld[2], nullptr, M, E_s(c),
+                          hx, hy, hz, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "16-bit encode kernel");
   uint32_t halo = 0;
   ST3D_CUDA(cudaMemcpyAsync(&halo, c->halo_max, sizeof halo, cudaMemcpyDeviceToHost, c->stream));
   ST3D_CUDA(cudaStreamSynchronize(c->stream));
   if (halo != 0)
     return fail(ST3D_ERR_UNSUPPORTED,
-                "16-bit storage needs a zero halo (a zero Dirichlet boundary); %s has nonzero halo values",
-                what);
+                "16-bit storage needs a zero halo (a zero Dirichlet boundary); s has nonzero halo values");
   return ST3D_OK;
 }
 
@@ -851,17 +850,41 @@ int delta_rebuild_pair(st3d_ctx* c) {
   return ST3D_OK;
 }
 
-// U from slot 0 (when u changed) and D from slot 0 - slot 1.
-int delta_encode_pair(st3d_ctx* c, bool u_changed) {
-  int rc;
+// U from slot 0 (when u changed) and D from slot 0 - slot 1.  `u` and `v`:
+// device arrays that the first pass reads in place of the slots and copies there.
+int delta_encode_pair(st3d_ctx* c, bool u_changed, const float* u = nullptr, const float* v = nullptr) {
   c->pair_valid = false;
-  if (u_changed &&
-      (rc = encode_staged16(c, stage_slot(c, 0), nullptr, c->fld[c->ub], Mu_buf(c, c->ub),
-                            Eu_buf(c, c->ub), "u", c->pair ? c->lo[c->ub] : nullptr)) != ST3D_OK)
-    return rc;
-  if ((rc = encode_staged16(c, stage_slot(c, 0), stage_slot(c, 1), c->fld[3], Md_lvl(c, c->lvl),
-                            Ed_lvl(c, c->lvl), "u or v")) != ST3D_OK)
-    return rc;
+  const st3d_grid_desc& g = c->grid;
+  const RefGeom R = ref_geom(g);
+  const int hx = g.xh < 4 ? (int)g.xh : 4, hy = g.yh < 4 ? (int)g.yh : 4, hz = (int)g.zh;
+  float* const su = stage_slot(c, 0);
+  float* const sv = stage_slot(c, 1);
+  uint32_t *Mu = Mu_buf(c, c->ub), *Md = Md_lvl(c, c->lvl);
+  PairMax pm;
+  if (u_changed) pm.Ma = Mu;
+  if (u) pm.to = su;
+  if (v) pm.to2 = sv;
+  if (u_changed) ST3D_CUDA(cudaMemsetAsync(Mu, 0, g.xs * sizeof(uint32_t), c->stream));
+  ST3D_CUDA(cudaMemsetAsync(Md, 0, g.xs * sizeof(uint32_t), c->stream));
+  ST3D_CUDA(cudaMemsetAsync(c->halo_max, 0, 2 * sizeof(uint32_t), c->stream));
+  cudaError_t e = launch_plane_max_ref(R, u ? u : su, Md, c->halo_max, hx, hy, hz, c->stream, v ? v : sv, pm);
+  if (e != cudaSuccess) return cuda_fail(e, "plane maximum kernel");
+  const int ws = word_storage(c->opts.storage);
+  uint16_t* d = (uint16_t*)c->fld[3];
+  if (u_changed)
+    e = launch_pair_to_dev16(ws, c->L, R, su, sv, (uint16_t*)c->fld[c->ub],
+                             c->pair ? (uint16_t*)c->lo[c->ub] : nullptr, d, Mu, Md, Eu_buf(c, c->ub),
+                             Ed_lvl(c, c->lvl), hx, hy, hz, c->stream);
+  else
+    e = launch_ref_to_dev16(ws, c->L, R, su, d, nullptr, Md, Ed_lvl(c, c->lvl), hx, hy, hz, c->stream, sv);
+  if (e != cudaSuccess) return cuda_fail(e, "16-bit encode kernel");
+  uint32_t halo[2] = {0, 0};
+  ST3D_CUDA(cudaMemcpyAsync(halo, c->halo_max, sizeof halo, cudaMemcpyDeviceToHost, c->stream));
+  ST3D_CUDA(cudaStreamSynchronize(c->stream));
+  if (halo[0] != 0 || halo[1] != 0)
+    return fail(ST3D_ERR_UNSUPPORTED,
+                "16-bit storage needs a zero halo (a zero Dirichlet boundary); %s has nonzero halo values",
+                halo[1] != 0 ? "u" : "u or v");
   c->pair_valid = true;
   return ST3D_OK;
 }
@@ -1351,13 +1374,13 @@ int upload_fields(st3d_ctx* c, const void* v, const void* s, const void* u) {
     if (u || v) {
       if (!(u && v) && !c->pair_valid && (rc = delta_rebuild_pair(c)) != ST3D_OK) return rc;
       c->pair_valid = false;
-      if (u)
-        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), u, host_array_bytes(c), cudaMemcpyDefault,
-                                  c->stream));
-      if (v)
-        ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 1), v, host_array_bytes(c), cudaMemcpyDefault,
-                                  c->stream));
-      if ((rc = delta_encode_pair(c, u != nullptr)) != ST3D_OK) return rc;
+      const size_t bytes = host_array_bytes(c);
+      const bool du = u && device_view(c, u, bytes), dv = v && device_view(c, v, bytes);
+      if (u && !du) ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), u, bytes, cudaMemcpyDefault, c->stream));
+      if (v && !dv) ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 1), v, bytes, cudaMemcpyDefault, c->stream));
+      if ((rc = delta_encode_pair(c, u != nullptr, du ? static_cast<const float*>(u) : nullptr,
+                                  dv ? static_cast<const float*>(v) : nullptr)) != ST3D_OK)
+        return rc;
       if (u) c->has_u = true;
       if (v) c->has_v = true;
     }
@@ -1369,9 +1392,7 @@ int upload_fields(st3d_ctx* c, const void* v, const void* s, const void* u) {
       else
         ST3D_CUDA(cudaMemcpyAsync(stage_slot(c, 0), s, host_array_bytes(c), cudaMemcpyDefault,
                                   c->stream));
-      if ((rc = encode_staged16(c, src, nullptr, c->fld[2], M_s(c), E_s(c), "s")) !=
-          ST3D_OK)
-        return rc;
+      if ((rc = encode_s16(c, src)) != ST3D_OK) return rc;
       c->has_s = true;
     }
     return ST3D_OK;
@@ -1702,7 +1723,7 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
       return cleanup(fail(ST3D_ERR_CUDA, "cudaMemsetAsync failed"));
   if (nbuf == 5) {
     if (cudaMalloc(&c->M, grid->xs * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&c->halo_max, sizeof(uint32_t)) != cudaSuccess) {
+        cudaMalloc(&c->halo_max, 2 * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
       return cleanup(fail(ST3D_ERR_NOMEM, "cudaMalloc of the halo check buffers failed"));
     }
@@ -1727,7 +1748,7 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
       }
     okm = okm && cudaMalloc(&c->E, 5 * xs * sizeof(int)) == cudaSuccess &&
           cudaMalloc(&c->M, 5 * xs * sizeof(uint32_t)) == cudaSuccess &&
-          cudaMalloc(&c->halo_max, sizeof(uint32_t)) == cudaSuccess;
+          cudaMalloc(&c->halo_max, 2 * sizeof(uint32_t)) == cudaSuccess;
     if (!okm) {
       cudaGetLastError();
       return cleanup(fail(ST3D_ERR_NOMEM, "cudaMalloc of the 16-bit storage buffers failed"));
@@ -2164,7 +2185,7 @@ int st3d_fill(st3d_ctx* c, int field, int kind, uint64_t seed, double a, double 
                                 bp, nb, 1, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "fill kernel launch");
     if (field == ST3D_FIELD_S)
-      rc = encode_staged16(c, stage_slot(c, 0), nullptr, c->fld[2], M_s(c), E_s(c), "s");
+      rc = encode_s16(c, stage_slot(c, 0));
     else
       rc = delta_encode_pair(c, field == ST3D_FIELD_U);
     if (rc != ST3D_OK) return rc;

@@ -313,15 +313,24 @@ cudaError_t launch_tma16(int storage, int points, const Tma16Plan& pl, const Geo
 
 // 16-bit storage transfers (st3d_kernels_copy.cu).
 // With `stage2`, the field is stage - stage2 (FP32) and the halo check
-// covers both arrays.
+// covers both arrays.  `pair`: the maxima of |stage| into Ma (its halo's into
+// halo_max[1]), copies of the points read into to / to2.
+struct PairMax {
+  uint32_t* Ma = nullptr;
+  float *to = nullptr, *to2 = nullptr;
+};
 cudaError_t launch_plane_max_ref(const RefGeom& R, const float* stage, uint32_t* M,
                                  uint32_t* halo_max, int hx, int hy, int hz, cudaStream_t stream,
-                                 const float* stage2 = nullptr);
-// With `lo16` (F16 words only), also the lo words of the FP16 hi/lo pair.
+                                 const float* stage2 = nullptr, const PairMax& pair = PairMax());
+// U of `stage` (with `ulo`, F16 words only, also the lo words of the FP16 hi/lo
+// pair) and D of stage - stage2 in one pass.
+cudaError_t launch_pair_to_dev16(int storage, const Layout& L, const RefGeom& R, const float* stage,
+                                 const float* stage2, uint16_t* uhi, uint16_t* ulo, uint16_t* dw,
+                                 const uint32_t* Mu, const uint32_t* Md, int* Eu, int* Ed, int hx, int hy,
+                                 int hz, cudaStream_t stream);
 cudaError_t launch_ref_to_dev16(int storage, const Layout& L, const RefGeom& R, const float* stage,
                                 uint16_t* hi, int8_t* lo, const uint32_t* M, int* E, int hx, int hy,
-                                int hz, cudaStream_t stream, const float* stage2 = nullptr,
-                                uint16_t* lo16 = nullptr);
+                                int hz, cudaStream_t stream, const float* stage2 = nullptr);
 // Delta form -> reference layout: u = dec(U) (minus_d false) or
 // v = dec(U) - dec(D) (minus_d true), interior rows with their k halo.
 // With `ul` (the F16_HL form) u = (U + ul) * 2^Eu.

@@ -260,11 +260,15 @@ constexpr int kMaxUnroll = 16;
 
 // Per-plane maxima of |x| over the interior (float bits, atomicMax) and the
 // maximum over the halo points the stencil reads; x = stage - stage2 when
-// stage2 is given (the halo check then covers both arrays).
+// stage2 is given (the halo check then covers both arrays).  With pair.Ma also
+// those of |stage| alone; with pair.to / to2 the points read go on into the
+// staging slots, so that a device array is read once for both (a copy of each
+// array and two passes over them took 1.3 ms more of a 1024^3 upload).
 template <int W>
 __global__ void __launch_bounds__(kCopyBlock)
     k_plane_max_ref(RefGeom R, const float* __restrict__ stage, const float* __restrict__ stage2,
-                    uint32_t* __restrict__ M, uint32_t* __restrict__ halo_max, int hx, int hy, int hz) {
+                    uint32_t* __restrict__ M, uint32_t* __restrict__ halo_max, PairMax pair, int hx, int hy,
+                    int hz) {
   const uint32_t kv = (uint32_t)(R.zs + 2 * hz) / W;
   const long long n = (long long)(R.ys + 2 * hy) * kv;
   const long long first = (long long)blockIdx.x * (kCopyBlock * kMaxUnroll);
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kCopyBlock)
   const RowRun run(first, kv);
   const long long plane = R.ijk_ofs + (long long)i * R.imult - (long long)hy * R.jmult - hz;
   const bool in_plane = i >= 0 && i < R.xs;
-  uint32_t m_in = 0u, m_halo = 0u;
+  uint32_t m_in = 0u, m_a = 0u, m_halo = 0u, m_halo_a = 0u;
 #pragma unroll 4
   for (int m = 0; m < kMaxUnroll; ++m) {
     const uint32_t y = threadIdx.x + m * kCopyBlock;
@@ -289,33 +293,92 @@ __global__ void __launch_bounds__(kCopyBlock)
 #pragma unroll
       for (int c = 0; c < W; ++c) b.x[c] = 0.0f;
     }
+    if (pair.to) store_floats<W>(pair.to + s, a);
+    if (pair.to2) store_floats<W>(pair.to2 + s, b);
     const bool in_row = in_plane && row >= hy && row < hy + R.ys;
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       const int k = (int)(word * W) + c - hz;
-      if (in_row && k >= 0 && k < R.zs)
+      const uint32_t ma = __float_as_uint(fabsf(a.x[c]));
+      if (in_row && k >= 0 && k < R.zs) {
         m_in = max(m_in, __float_as_uint(fabsf(a.x[c] - b.x[c])));
-      else
+        m_a = max(m_a, ma);
+      } else {
         m_halo = max(m_halo, __float_as_uint(fmaxf(fabsf(a.x[c]), fabsf(b.x[c]))));
+        m_halo_a = max(m_halo_a, ma);
+      }
     }
   }
   const uint32_t a = __reduce_max_sync(0xffffffffu, m_in);
   const uint32_t b = __reduce_max_sync(0xffffffffu, m_halo);
-  if ((threadIdx.x & 31) == 0) {
+  const bool lead = (threadIdx.x & 31) == 0;
+  if (lead) {
     if (a && in_plane) atomicMax(&M[i], a);
     if (b) atomicMax(halo_max, b);
+  }
+  if (pair.Ma) {
+    const uint32_t ua = __reduce_max_sync(0xffffffffu, m_a);
+    const uint32_t ub = __reduce_max_sync(0xffffffffu, m_halo_a);
+    if (lead && ua && in_plane) atomicMax(&pair.Ma[i], ua);
+    if (lead && ub) atomicMax(halo_max + 1, ub);
+  }
+}
+
+// U from stage (with ulo the lo words of the hi/lo pair too, fp16(xs - hi)) and
+// D = stage - stage2 in one pass over the slots: what k_ref_to_dev16 writes for each.
+template <int KIND, int W>
+__global__ void __launch_bounds__(kCopyBlock)
+    k_pair_to_dev16(Layout L, RefGeom R, const float* __restrict__ stage, const float* __restrict__ stage2,
+                    uint16_t* __restrict__ uhi, uint16_t* __restrict__ ulo, uint16_t* __restrict__ dw,
+                    const uint32_t* __restrict__ Mu, const uint32_t* __restrict__ Md, int* __restrict__ Eu,
+                    int* __restrict__ Ed, int hx, int hy, int hz) {
+  const uint32_t kv = (uint32_t)(R.zs + 2 * hz) / W;
+  const long long n = (long long)(R.ys + 2 * hy) * kv;
+  const long long first = (long long)blockIdx.x * (kCopyBlock * kCopyUnroll);
+  const int i = (int)blockIdx.y - hx;
+  const RowRun run(first, kv);
+  const bool plane_in = i >= 0 && i < R.xs;
+  const int eu = plane_in ? scale_exponent(__uint_as_float(Mu[i])) : 0;
+  const int ed = plane_in ? scale_exponent(__uint_as_float(Md[i])) : 0;
+  if (plane_in && blockIdx.x == 0 && threadIdx.x == 0) {
+    Eu[i] = eu;
+    Ed[i] = ed;
+  }
+  const float inv_u = exp2i(-eu), inv_d = exp2i(-ed);
+  const long long splane = R.ijk_ofs + (long long)i * R.imult - (long long)hy * R.jmult - hz;
+  const long long dplane =
+      ((long long)(i + (int)L.pi) * L.nj + ((int)L.pj - hy)) * L.nk + (int)L.pk - hz;
+#pragma unroll
+  for (int m = 0; m < kCopyUnroll; ++m) {
+    const uint32_t y = threadIdx.x + m * kCopyBlock;
+    if (first + y >= n) break;
+    long long row;
+    uint32_t word;
+    run.at(y, &row, &word);
+    const long long s = splane + row * R.jmult + (long long)word * W;
+    const long long d = dplane + row * (long long)L.nk + (long long)word * W;
+    const Floats<W> a = load_floats<W>(stage + s), b = load_floats<W>(stage2 + s);
+    Words<W> h, l, q;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+      const float xs = a.x[c] * inv_u;
+      h.w[c] = float_to_word<KIND>(xs);
+      l.w[c] = float_to_word<KIND>(xs - word_to_float<KIND>(h.w[c]));
+      q.w[c] = float_to_word<KIND>((a.x[c] - b.x[c]) * inv_d);
+    }
+    store_words<W>(uhi + d, h);
+    if (ulo) store_words<W>(ulo + d, l);
+    store_words<W>(dw + d, q);
   }
 }
 
 // Scatter + encode: staging (reference layout, float) -> words (+ low bytes)
 // in the library layout, the plane's scale from its maximum.
-// With lo16 (FP16 words), the lo word of the hi/lo pair: fp16(xs - hi).
 template <int KIND, bool HILO, int W>
 __global__ void __launch_bounds__(kCopyBlock)
     k_ref_to_dev16(Layout L, RefGeom R, const float* __restrict__ stage,
                    const float* __restrict__ stage2, uint16_t* __restrict__ hi, int8_t* __restrict__ lo,
-                   const uint32_t* __restrict__ M, int* __restrict__ E, int hx, int hy, int hz,
-                   uint16_t* __restrict__ lo16) {
+                   const uint32_t* __restrict__ M, int* __restrict__ E, int hx, int hy, int hz) {
   const uint32_t kv = (uint32_t)(R.zs + 2 * hz) / W;
   const long long n = (long long)(R.ys + 2 * hy) * kv;
   const long long first = (long long)blockIdx.x * (kCopyBlock * kCopyUnroll);
@@ -343,7 +406,7 @@ __global__ void __launch_bounds__(kCopyBlock)
 #pragma unroll
       for (int c = 0; c < W; ++c) x.x[c] = x.x[c] - b.x[c];
     }
-    Words<W> h, l;
+    Words<W> h;
     int8_t q8[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
@@ -351,7 +414,6 @@ __global__ void __launch_bounds__(kCopyBlock)
       const uint16_t w = float_to_word<KIND>(xs);
       const float r = xs - word_to_float<KIND>(w);
       h.w[c] = w;
-      l.w[c] = float_to_word<KIND>(r);
       if (HILO) {
         int eb = (w >> 10) & 0x1f;
         if (eb == 0) eb = 1;
@@ -361,7 +423,6 @@ __global__ void __launch_bounds__(kCopyBlock)
       }
     }
     store_words<W>(hi + d, h);
-    if (lo16) store_words<W>(lo16 + d, l);
     if (HILO) {
       if constexpr (W == 4) {
         *reinterpret_cast<char4*>(lo + d) = make_char4(q8[0], q8[1], q8[2], q8[3]);
@@ -460,37 +521,64 @@ dim3 max_grid(long long rows, long long klen, int W, unsigned planes) {
 
 cudaError_t launch_plane_max_ref(const RefGeom& R, const float* stage, uint32_t* M,
                                  uint32_t* halo_max, int hx, int hy, int hz, cudaStream_t stream,
-                                 const float* stage2) {
+                                 const float* stage2, const PairMax& pair) {
   const unsigned planes = (unsigned)(R.xs + 2 * hx);
   const long long rows = R.ys + 2 * hy, klen = R.zs + 2 * hz;
   if (planes > 65535) return cudaErrorInvalidConfiguration;
-  const uintptr_t at = reinterpret_cast<uintptr_t>(stage) | reinterpret_cast<uintptr_t>(stage2);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(stage) | reinterpret_cast<uintptr_t>(stage2) |
+                       reinterpret_cast<uintptr_t>(pair.to) | reinterpret_cast<uintptr_t>(pair.to2);
   if (R.jmult % 4 == 0 && R.ijk_ofs % 4 == hz % 4 && klen % 4 == 0 && at % 16 == 0)
     k_plane_max_ref<4><<<max_grid(rows, klen, 4, planes), kCopyBlock, 0, stream>>>(R, stage, stage2, M, halo_max,
-                                                                                   hx, hy, hz);
+                                                                                   pair, hx, hy, hz);
   else
     k_plane_max_ref<1><<<max_grid(rows, klen, 1, planes), kCopyBlock, 0, stream>>>(R, stage, stage2, M, halo_max,
-                                                                                   hx, hy, hz);
+                                                                                   pair, hx, hy, hz);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pair_to_dev16(int storage, const Layout& L, const RefGeom& R, const float* stage,
+                                 const float* stage2, uint16_t* uhi, uint16_t* ulo, uint16_t* dw,
+                                 const uint32_t* Mu, const uint32_t* Md, int* Eu, int* Ed, int hx, int hy,
+                                 int hz, cudaStream_t stream) {
+  const unsigned planes = (unsigned)(R.xs + 2 * hx);
+  const long long rows = R.ys + 2 * hy, klen = R.zs + 2 * hz;
+  if (planes > 65535) return cudaErrorInvalidConfiguration;
+  if (ulo && storage != ST3D_F16) return cudaErrorInvalidValue;
+  const bool fours = rows_in_fours(L, R, hz, stage, stage2);
+  const dim3 grid = run_grid(rows, klen, fours ? 4 : 1, planes);
+#define ST3D_ENCODE(KIND, W)                                                                          \
+  k_pair_to_dev16<KIND, W><<<grid, kCopyBlock, 0, stream>>>(L, R, stage, stage2, uhi, ulo, dw, Mu, Md, \
+                                                            Eu, Ed, hx, hy, hz)
+  if (storage == ST3D_F16 && fours)
+    ST3D_ENCODE(0, 4);
+  else if (storage == ST3D_F16)
+    ST3D_ENCODE(0, 1);
+  else if (storage == ST3D_BF16 && fours)
+    ST3D_ENCODE(1, 4);
+  else if (storage == ST3D_BF16)
+    ST3D_ENCODE(1, 1);
+  else
+    return cudaErrorInvalidValue;
+#undef ST3D_ENCODE
   return cudaGetLastError();
 }
 
 cudaError_t launch_ref_to_dev16(int storage, const Layout& L, const RefGeom& R, const float* stage,
                                 uint16_t* hi, int8_t* lo, const uint32_t* M, int* E, int hx, int hy,
-                                int hz, cudaStream_t stream, const float* stage2, uint16_t* lo16) {
+                                int hz, cudaStream_t stream, const float* stage2) {
   const unsigned planes = (unsigned)(R.xs + 2 * hx);
   const long long rows = R.ys + 2 * hy, klen = R.zs + 2 * hz;
   if (planes > 65535) return cudaErrorInvalidConfiguration;
-  if (lo16 && storage != ST3D_F16) return cudaErrorInvalidValue;
   const bool fours = rows_in_fours(L, R, hz, stage, stage2);
   const dim3 grid = run_grid(rows, klen, fours ? 4 : 1, planes);
 #define ST3D_ENCODE(KIND, HILO)                                                                       \
   do {                                                                                                \
     if (fours)                                                                                        \
       k_ref_to_dev16<KIND, HILO, 4><<<grid, kCopyBlock, 0, stream>>>(L, R, stage, stage2, hi, lo, M,  \
-                                                                     E, hx, hy, hz, lo16);            \
+                                                                     E, hx, hy, hz);                  \
     else                                                                                              \
       k_ref_to_dev16<KIND, HILO, 1><<<grid, kCopyBlock, 0, stream>>>(L, R, stage, stage2, hi, lo, M,  \
-                                                                     E, hx, hy, hz, lo16);            \
+                                                                     E, hx, hy, hz);                  \
   } while (0)
   if (storage == ST3D_F16)
     ST3D_ENCODE(0, false);

@@ -85,3 +85,48 @@ def test_device_arrays_in_16_bit_storage(grid, shift, storage):
         assert api.lib().st3d_upload(b.handle, None, None, p(bad)) == S.api.ERR_UNSUPPORTED
     np.testing.assert_array_equal(out[0].cpu().numpy(), hv)
     np.testing.assert_array_equal(out[1].cpu().numpy(), hu)
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16_hl"])
+@pytest.mark.parametrize("grid", [(5, 9, 64, 4, 4, 4), (3, 40, 61, 5, 5, 5)])
+def test_one_device_array_of_the_pair(grid, storage):
+    """u or v alone: the other's values come from an earlier upload (then from
+    the device state once a step was taken); a halo point of either is named."""
+    torch = pytest.importorskip("torch")
+    g = S.Grid(*grid)
+    fields = []
+    for f in range(5):
+        a = np.zeros(O.shape(grid), np.float32)
+        O.interior(a, grid)[...] = O.interior(O.fill_uniform(grid, 5, f, -3.0, 3.0), grid)
+        fields.append(a)
+    dev = [_device(a, 0) for a in fields]
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    up, err = api.lib().st3d_upload, S.api.ERR_UNSUPPORTED
+    got = []
+    with S.Stencil(g, 7, "wave", storage, dt=1e-3) as a, S.Stencil(g, 7, "wave", storage, dt=1e-3) as b:
+        for st, arr in ((a, [x.ctypes.data_as(C.c_void_p) for x in fields]), (b, [p(t) for t in dev])):
+            assert up(st.handle, arr[0], arr[1], arr[2]) == 0
+            assert up(st.handle, None, None, arr[3]) == 0
+            assert up(st.handle, arr[4], None, None) == 0
+            st.iterate(3)
+            assert up(st.handle, None, None, arr[0]) == 0
+            st.iterate(2)
+            hv, hu = np.zeros_like(fields[0]), np.zeros_like(fields[0])
+            st.download(hv, hu)
+            st.synchronize()
+            got.append((hv, hu))
+        for which, name in ((0, "u or v"), (2, "u")):
+            bad = dev[which].clone()
+            bad.view(-1)[bad.numel() // 2] = 1.0  # a k halo point where zs is even, an inner one else
+            i, j, k = np.unravel_index(bad.numel() // 2, fields[0].shape)
+            inner = all(grid[3 + x] <= q < grid[3 + x] + grid[x] for x, q in enumerate((i, j, k)))
+            if inner:
+                bad.view(-1)[bad.numel() // 2 - k] = 1.0
+            torch.cuda.synchronize()
+            args = [None, None, None]
+            args[which] = p(bad)
+            assert up(b.handle, *args) == err
+            assert ("; %s has" % name) in S.last_error()
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)
