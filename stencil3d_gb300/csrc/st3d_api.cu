@@ -632,8 +632,9 @@ double mma_step_us(bool tall, int points, bool pair) {
 // time above; WIDE where the request names a tile height or depth.  Measured,
 // us a step WIDE and TALL: FP16 25 points 512^3 326 / 290 (492 tile steps either
 // way; 1024^3, 3096 against 3672, stays WIDE: 2085), 7 points 512^3 272 / 234,
-// 1024^3 1785 / 1720; F16_HL 25 points 512^3 396 / 324, 1024^3 2686 / 2425, 13
-// points 512^3 388 / 306; the worst met, F16_HL 7 points 200 x 700 x 500, 205 / 208.
+// 1024^3 1785 / 1720; F16_HL 25 points 512^3 396 / 324, 1024^3 2710 / 2425 to
+// 2700 between runs, 13 points 512^3 388 / 306; the worst met, F16_HL 7 points
+// 200 x 700 x 500, 205 / 208.
 int plan_mma16(st3d_ctx* c, int sm_count, int max_smem) {
   Tma16Plan* p = new (std::nothrow) Tma16Plan();
   if (!p) return fail(ST3D_ERR_NOMEM, "host allocation failed");
