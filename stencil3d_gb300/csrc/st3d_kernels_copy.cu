@@ -25,14 +25,20 @@ namespace {
 
 // A transfer works on planes: blockIdx.y is the plane, and the plane's rows
 // (each `kv` words of W points, halos included) form one flat run that the
-// blocks cut into pieces of kCopyBlock * kCopyUnroll words, so short rows fill
+// blocks cut into pieces of kCopyBlock * kRunUnroll words, so short rows fill
 // the blocks as well as long ones (one block a row left 3/4 of the threads
-// idle on 200-point rows).  A thread moves kCopyUnroll words, loads first:
+// idle on 200-point rows).  A thread moves kRunUnroll words, loads first:
 // bound by HBM (1024^3 FP32, 16-byte words: 1.45 ms an array, 6.0 TB/s,
 // against 1.70 ms for one block a row with 4-byte words) or by the host link,
 // which needs several transfers in flight per thread.
 constexpr int kCopyUnroll = 4;
 constexpr int kCopyBlock = 256;
+// Rows that are not whole 16-byte words move element by element, twice as many
+// a thread: with four the bytes in flight bound them (525 x 219 x 387 FP32 device
+// array, up / down: 4 elements 4110 / 4047 GB/s, 8 5171 / 5121, 12 5491 / 5074,
+// 16 5527 / 4533).
+template <int W>
+constexpr int kRunUnroll = W == 1 ? 2 * kCopyUnroll : kCopyUnroll;
 
 // Row and word of the flat run's element `first + m`, the block's first
 // element split once into (row, rest).
@@ -70,18 +76,19 @@ __device__ __forceinline__ int line_shift(const V* p) {
 template <typename V, int W, bool UP>
 __device__ __forceinline__ void copy_plane_piece(const Layout& L, const RefGeom& R, V* dev, V* ref, int i, int hy,
                                                  int hz) {
+  constexpr int U = kRunUnroll<W>;
   const uint32_t kv = (uint32_t)(R.zs + 2 * hz) / W;
   const long long n = (long long)(R.ys + 2 * hy) * kv;
   V* span = ref + (R.ijk_ofs + (long long)i * R.imult - (long long)hy * R.jmult - hz) / W;
   V* plane = dev + (((long long)(i + (int)L.pi) * L.nj + ((int)L.pj - hy)) * L.nk + (int)L.pk - hz) / W;
-  const long long at = (long long)blockIdx.x * (kCopyBlock * kCopyUnroll) - line_shift(span);
+  const long long at = (long long)blockIdx.x * (kCopyBlock * U) - line_shift(span);
   const long long first = at > 0 ? at : 0;
   const int lead = (int)(first - at);
   const RowRun run(first, kv);
-  V x[kCopyUnroll];
-  long long to[kCopyUnroll];
+  V x[U];
+  long long to[U];
 #pragma unroll
-  for (int m = 0; m < kCopyUnroll; ++m) {
+  for (int m = 0; m < U; ++m) {
     const int y = (int)threadIdx.x + m * kCopyBlock - lead;
     to[m] = -1;
     if (y >= 0 && first + y < n) {
@@ -99,7 +106,7 @@ __device__ __forceinline__ void copy_plane_piece(const Layout& L, const RefGeom&
     }
   }
 #pragma unroll
-  for (int m = 0; m < kCopyUnroll; ++m)
+  for (int m = 0; m < U; ++m)
     if (to[m] >= 0) (UP ? plane : span)[to[m]] = x[m];
 }
 
@@ -125,8 +132,8 @@ bool rows_in_words(int W, const Layout& L, const RefGeom& R, int hz, const void*
          (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 == 0;
 }
 
-dim3 run_grid(long long rows, long long klen, int W, unsigned planes) {
-  const long long piece = kCopyBlock * kCopyUnroll, shift = 31;  // words a piece may be shifted by
+dim3 run_grid(long long rows, long long klen, int W, unsigned planes, int unroll = kCopyUnroll) {
+  const long long piece = kCopyBlock * unroll, shift = 31;  // words a piece may be shifted by
   return dim3((unsigned)((rows * (klen / W) + shift + piece - 1) / piece), planes, 1);
 }
 
@@ -146,7 +153,7 @@ cudaError_t launch_ref_to_dev(int eb, const Layout& L, const RefGeom& R, const v
     else
       k_ref_to_dev<double2, 2><<<grid, kCopyBlock, 0, stream>>>(L, R, (const double2*)stage, (double2*)dst, hx, hy, hz);
   } else {
-    const dim3 grid = run_grid(rows, klen, 1, planes);
+    const dim3 grid = run_grid(rows, klen, 1, planes, kRunUnroll<1>);
     if (eb == 4)
       k_ref_to_dev<float, 1><<<grid, kCopyBlock, 0, stream>>>(L, R, (const float*)stage, (float*)dst, hx, hy, hz);
     else
@@ -169,7 +176,7 @@ cudaError_t launch_dev_to_ref(int eb, const Layout& L, const RefGeom& R, const v
     else
       k_dev_to_ref<double2, 2><<<grid, kCopyBlock, 0, stream>>>(L, R, (const double2*)src, (double2*)stage, hz);
   } else {
-    const dim3 grid = run_grid(rows, klen, 1, planes);
+    const dim3 grid = run_grid(rows, klen, 1, planes, kRunUnroll<1>);
     if (eb == 4)
       k_dev_to_ref<float, 1><<<grid, kCopyBlock, 0, stream>>>(L, R, (const float*)src, (float*)stage, hz);
     else
