@@ -306,13 +306,12 @@ __global__ void __launch_bounds__(kCopyBlock)
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       const int k = (int)(word * W) + c - hz;
-      const uint32_t ma = __float_as_uint(fabsf(a.x[c]));
       if (in_row && k >= 0 && k < R.zs) {
         m_in = max(m_in, __float_as_uint(fabsf(a.x[c] - b.x[c])));
-        m_a = max(m_a, ma);
+        m_a = max(m_a, __float_as_uint(fabsf(a.x[c])));
       } else {
         m_halo = max(m_halo, __float_as_uint(fmaxf(fabsf(a.x[c]), fabsf(b.x[c]))));
-        m_halo_a = max(m_halo_a, ma);
+        m_halo_a = max(m_halo_a, __float_as_uint(fmaxf(fabsf(a.x[c]), 0.0f)));  // a NaN passes, as in m_halo
       }
     }
   }

@@ -128,5 +128,13 @@ def test_one_device_array_of_the_pair(grid, storage):
             args[which] = p(bad)
             assert up(b.handle, *args) == err
             assert ("; %s has" % name) in S.last_error()
+    # a NaN is no halo value to refuse, on either route
+    host = fields[2].copy()
+    host.reshape(-1)[0] = np.nan
+    nan = _device(host, 0)
+    torch.cuda.synchronize()
+    for u in (host.ctypes.data_as(C.c_void_p), p(nan)):
+        with S.Stencil(g, 7, "wave", storage, dt=1e-3) as st:
+            assert up(st.handle, p(dev[0]), p(dev[1]), u) == 0
     for x, y in zip(*got):
         np.testing.assert_array_equal(x, y)
