@@ -87,8 +87,9 @@ struct Twice {
 ST3D_HD Twice twice_of(double u) {
   const Bits64 b = bits_of(u);
   Twice t;
-  const int e = (int)(b.hi & kExpMask);
-  t.e = e ? e + kExpOne : 0;  // zero and subnormal u fail the range check
+  const uint32_t e = b.hi & kExpMask;
+  // 0, which fails the range check, for zero and subnormal u and where 2u is not finite
+  t.e = e - kExpOne < 2045u * kExpOne ? (int)(e + kExpOne) : 0;
   t.hi = (b.hi & 0xfffffu) | 0x100000u;
   t.lo = b.lo;
   t.neg = ~(uint32_t)((int32_t)b.hi >> 31);
