@@ -87,7 +87,9 @@ __global__ void __launch_bounds__(kSimpleBX* kSimpleBY)
         lap = p == 0 ? cf.cf[0] * d : fma_t<T>(cf.cf[p], d, lap);
       }
       if (i == src_i && j == src_j && k == src_k) s0 = s0 + amp;
-      T t = fma_t<T>(T(2), u0, -v0);  // 2u - v, rounded once as the difference is
+      // 2u - v in one multiply-add, rounded once as the difference is; where 2u
+      // overflows it has to be infinite first (u of exponent 2046 and above)
+      T t = (bits_of(u0).hi & 0x7fe00000u) == 0x7fe00000u ? (u0 + u0) - v0 : fma_t<T>(T(2), u0, -v0);
       t = fma_t<T>(cf.c1, lap, t);
       v[x] = fma_t<T>(cf.c2, s0, t);
 #pragma unroll
