@@ -1179,6 +1179,45 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
   return ST3D_OK;
 }
 
+// Time of n wave steps of a call as the launches st3d_iterate makes of them, us.
+double steps_us(const st3d_ctx* c, uint32_t n) {
+  double us = 0.0;
+  while (n > 0) {
+    uint32_t many = std::min(n, (uint32_t)kWaveSteps);
+    if (c->brick.nbi > 0) {
+      us += brick_us(c->brick, c->R, (int)many);
+    } else {
+      many = std::min(many, (uint32_t)c->wave->max_steps);
+      WavePlan w;
+      double part = 0.0;
+      us += plan_wave(c, many, &w, &part) ? part : many * single_step_us(c);
+    }
+    n -= many;
+  }
+  return us;
+}
+
+// Whether a wave call of more steps than the pipeline of levels takes
+// (iterate_host_wave) runs faster over chunks of planes beside its transfers
+// (st3d_stream.cu) or phase by phase, the steps many a launch with all CTAs.
+// Chunks hide the downloads and most of the uploads, but step slower: an item
+// (16 planes of a tile) takes 11 / 11.6 / 14.3 us at 7 / 13 / 25 points on about 108
+// CTAs, and a (step, chunk) waits for the one before, so fewer tiles than CTAs
+// leave CTAs idle.  Pinned arrays, ms a call in chunks / in phases: 7 points 512^3
+// 33 steps 19.5 / 21.3, 48 steps 25.7 / 24.6; 1024^3 33 steps 122 / 173, 64 steps
+// 215 / 227, 100 steps 324 / 294; 25 points 1024^3 33 steps 140 / 185, 100 steps
+// 379 / 335; 768^3 33 steps 70.4 / 77.9, 48 steps 99.2 / 91.5; up to 384^3 phases
+// (33 steps 10.2 / 9.3).  Over 64^3 to 1024^3, three orders and 33 to 250 steps
+// the choice is at most 5 % behind the better of the two.
+bool chunks_faster(const st3d_ctx* c, uint32_t iterations) {
+  const double bytes = (double)host_array_bytes(c);
+  const double up = 3.0 * bytes / 211e3, down = 2.0 * bytes / 194e3;  // the link's rates
+  const double item = c->R == 1 ? 11.0 : c->R == 2 ? 11.6 : 14.3;
+  const double chunks = (double)((c->grid.xs + 15) / 16), tiles = (double)c->tma->ntj * c->tma->ntk;
+  return 0.2 * up + iterations * chunks * item * std::max(1.0, tiles / 108.0) <
+         up + down + steps_us(c, iterations);
+}
+
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and
 // download in one cooperative launch.  *done = false (and nothing enqueued)
 // where it does not apply; the caller then runs the phases one by one.
@@ -1197,11 +1236,8 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   const float* hs = static_cast<const float*>(direct_view(s, hbytes));
   const float* hu = static_cast<const float*>(direct_view(u, hbytes));
   if (!hv || !hs || !hu) return ST3D_OK;
-  // many wave steps run better between the transfers than beside them (L2 or
-  // shared memory for all CTAs): 7 points 512^3, 200 steps 72 ms streamed, 60
-  // phase by phase; 64^3, 100 steps 0.98 and 0.32
-  if (c->opts.mode == ST3D_MODE_WAVE && iterations > (uint32_t)kWaveLevels &&
-      (c->wave || c->brick.nbi > 0))
+  if (hp == ST3D_HOST_AUTO && c->opts.mode == ST3D_MODE_WAVE && iterations > (uint32_t)kWaveLevels &&
+      (c->wave || c->brick.nbi > 0) && !chunks_faster(c, iterations))
     return ST3D_OK;
   if (c->wave) {
     const int rc = iterate_host_wave(c, const_cast<float*>(hv), hs, const_cast<float*>(hu), iterations, done);
