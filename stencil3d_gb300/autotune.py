@@ -57,13 +57,13 @@ def candidates(points, mode, storage, zero_halo=False):
     if storage == "f16_hilo":
         return [{"kernel": "tma", "tile_j": 16, "stages": nv} for nv in (4, 6, 8, 12)]
     if storage == "f64" or points == 2:
-        return [{"kernel": "simple", "ichunk": ic} for ic in (32, 64, 128)]
+        return [{"kernel": "simple", "ichunk": ic} for ic in (0, 32, 64, 128)]
     # FP32: the TMA pipeline shapes the kernel serves, a few unit lengths,
     # and the plain kernel as a floor
     for tj, nv in ((16, 4), (16, 3), (16, 2), (8, 4), (8, 3)):
         for ic in (0, 64, 256):
             out.append({"kernel": "tma", "tile_j": tj, "stages": nv, "ichunk": ic})
-    out.append({"kernel": "simple", "ichunk": 64})
+    out += [{"kernel": "simple", "ichunk": ic} for ic in (0, 64)]
     if mode == "wave":
         # the library's own choice, which may take several steps a launch (no
         # shape of the one-step kernel named)
