@@ -32,6 +32,9 @@ import time
 from . import api
 
 CACHE_ENV = "ST3D_TUNE_CACHE"
+# Part of every cache key: raised when the candidates or what they run change, so
+# that a choice made among others is not handed out again.
+CANDIDATES_VERSION = 2
 KNOBS = ("kernel", "tile_j", "stages", "ichunk", "temporal_block")
 
 
@@ -78,9 +81,9 @@ def candidates(points, mode, storage, zero_halo=False):
 
 def cache_key(grid, points, mode, storage, device=None):
     d = device if device is not None else api.device_info()
-    return "sm%d_cc%d%d|%d|%s|%s|%dx%dx%d|h%d,%d,%d" % (
+    return "sm%d_cc%d%d|%d|%s|%s|%dx%dx%d|h%d,%d,%d|c%d" % (
         d["sm_count"], d["cc"][0], d["cc"][1], points, mode, storage, grid.xsize, grid.ysize,
-        grid.zsize, grid.xhalo, grid.yhalo, grid.zhalo)
+        grid.zsize, grid.xhalo, grid.yhalo, grid.zhalo, CANDIDATES_VERSION)
 
 
 def load_cache(path):
@@ -132,7 +135,8 @@ def tune(grid, points, mode="wave", storage="f32", steps=10, cache=None, refresh
          zero_halo=False, measure=None, device=None, phys=None):
     """Best configuration for the workload: {"opts": overrides, "ms_per_step",
     "gpts", "table": [[candidate, ms], ...], "key"}.  The result is cached
-    under the workload's key (device, stencil, mode, storage, sizes, halos)."""
+    under the workload's key (device, stencil, mode, storage, sizes, halos, and
+    the version of the candidates)."""
     path = cache if cache is not None else default_cache_path()
     key = cache_key(grid, points, mode, storage, device)
     data = load_cache(path)
@@ -160,14 +164,15 @@ def tune(grid, points, mode="wave", storage="f32", steps=10, cache=None, refresh
 
 
 def batch_key(grids, points, device=None):
-    """Cache key of a batch: device, and a digest of the (sizes, halos,
-    order) list in order."""
+    """Cache key of a batch: device, a digest of the (sizes, halos, order)
+    list in order, and the version of the candidates."""
     import hashlib
     d = device if device is not None else api.device_info()
     desc = ";".join("%dx%dx%d|%d,%d,%d|%d" % (g.xsize, g.ysize, g.zsize, g.xhalo, g.yhalo, g.zhalo, p)
                     for g, p in zip(grids, points))
-    return "sm%d_cc%d%d|batch|%d|%s" % (d["sm_count"], d["cc"][0], d["cc"][1], len(grids),
-                                         hashlib.sha1(desc.encode()).hexdigest()[:16])
+    return "sm%d_cc%d%d|batch|%d|%s|c%d" % (d["sm_count"], d["cc"][0], d["cc"][1], len(grids),
+                                             hashlib.sha1(desc.encode()).hexdigest()[:16],
+                                             CANDIDATES_VERSION)
 
 
 def batch_candidates():

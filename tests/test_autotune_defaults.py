@@ -1,5 +1,7 @@
 """The tuners time the library's own choice beside the named ones, so that what
 they return is never slower than naming nothing."""
+import json
+
 import pytest
 
 import stencil3d_gb300 as S
@@ -31,3 +33,19 @@ def test_every_list_has_the_automatic_unit_length(points, mode, storage):
     cands = autotune.candidates(points, mode, storage)
     for kernel in {c["kernel"] for c in cands}:
         assert any(c["kernel"] == kernel and c.get("ichunk", 0) == 0 for c in cands), kernel
+
+
+def test_a_choice_among_older_candidates_is_not_reused(tmp_path):
+    """Cache files of before the version stood in the key: the workload is timed again."""
+    grid, path = S.Grid(256, 256, 256, 4, 4, 4), tmp_path / "t.json"
+    old = "sm152_cc103|25|wave|f32|256x256x256|h4,4,4"
+    stale = {"key": old, "opts": {"kernel": "tma", "tile_j": 16, "stages": 4, "ichunk": 0}, "ms_per_step": 9.0}
+    batch = "|".join(autotune.batch_key([grid], [7], DEV).split("|")[:4])
+    path.write_text(json.dumps({old: stale, batch: {"key": batch, "opts": {"ichunk": 512, "schedule": "persistent"}}}))
+    best = autotune.tune(grid, 25, cache=str(path), device=DEV,
+                         measure=lambda c: 1.0 if c == {"kernel": "tma"} else 2.0)
+    assert best["opts"] == {"kernel": "tma"}
+    best = autotune.tune_batch([grid], [7], cache=str(path), device=DEV,
+                               measure=lambda c: 1.0 if c["schedule"] == "graph" else 2.0)
+    assert best["opts"]["schedule"] == "graph"
+    assert old in json.loads(path.read_text())  # left where an older library finds it
