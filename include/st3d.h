@@ -154,7 +154,7 @@ typedef struct st3d_opts {
   int32_t pad0;
   double src_f, src_t0, dt;          /* Ricker peak frequency [Hz], delay [s], time step [s] */
   int32_t temporal_block;            /* mode W steps fused per pass: 1, 2 or 4 */
-  int32_t tile_j, tile_k;            /* CTA tile; 0 = automatic */
+  int32_t tile_j, tile_k;            /* CTA tile; 0 = automatic (the tensor-core kernel: 16 or 32 rows) */
   int32_t ichunk;                    /* planes per work unit along i; 0 = automatic */
   int32_t stages;                    /* pipeline stages of the TMA kernels; 0 = automatic */
   int32_t host_path;                 /* st3d_host_path of FP32/FP64 uploads and downloads */

@@ -137,6 +137,21 @@ template Coefs<double> make_coefs<double>(const st3d_opts&);
 
 namespace {
 
+// The tensor-core kernel serves a delta-form request when asked for, or under
+// ST3D_KERNEL_AUTO when the request names no tile height or pipeline depth of
+// the scalar kernel, or the height (32) that only this one has: measured at
+// 1024^3 on a GB300 it is the faster kernel of the delta forms (25 points FP16
+// 515 against 317 Gpts/s, BF16 498 / 312, F16_HL 397 / 283; 13 points (1040^3)
+// FP16 500 / 408, F16_HL 410 / 363; 7 points FP16 615 / 545, BF16 603 / 531,
+// F16_HL 418 / 357).
+bool mma_chosen(const st3d_opts& o) {
+  const bool delta = o.storage == ST3D_F16 || o.storage == ST3D_BF16 || o.storage == ST3D_F16_HL;
+  if (!delta || o.mode != ST3D_MODE_WAVE) return false;
+  if (o.kernel == ST3D_KERNEL_MMA) return true;
+  return o.kernel == ST3D_KERNEL_AUTO &&
+         (o.tile_j == MmaTile<true>::TJ || (o.tile_j == 0 && o.stages == 0));
+}
+
 int validate(const st3d_grid_desc* g, const st3d_opts* o) {
   if (!g || !o) return fail(ST3D_ERR_INVALID, "null grid or options");
   const int R = radius_of(o->points);
@@ -167,16 +182,17 @@ int validate(const st3d_grid_desc* g, const st3d_opts* o) {
   const bool delta16 = o->storage == ST3D_F16 || o->storage == ST3D_BF16 || o->storage == ST3D_F16_HL;
   if (o->kernel == ST3D_KERNEL_MMA && !delta16)
     return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel serves the 16-bit delta forms (F16, BF16, F16_HL)");
-  if (o->kernel == ST3D_KERNEL_MMA && o->tile_j != 0 && o->tile_j != 16)
-    return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel runs 16-row tiles, not %d", o->tile_j);
-  if (o->kernel == ST3D_KERNEL_MMA && o->stages != 0 && o->stages != (o->storage == ST3D_F16_HL ? 4 : 8))
-    return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel runs %d stages, not %d",
-                o->storage == ST3D_F16_HL ? 4 : 8, o->stages);
+  const bool mma = mma_chosen(*o);
+  if (mma && o->tile_j != 0 && o->tile_j != MmaTile<false>::TJ && o->tile_j != MmaTile<true>::TJ)
+    return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel runs 16- and 32-row tiles, not %d", o->tile_j);
+  const int depth = o->storage == ST3D_F16_HL && o->tile_j != MmaTile<true>::TJ ? 4 : 8;
+  if (mma && o->stages != 0 && o->stages != depth)
+    return fail(ST3D_ERR_UNSUPPORTED, "the tensor-core kernel runs %d stages, not %d", depth, o->stages);
   if (o->kernel == ST3D_KERNEL_TMA && o->storage == ST3D_F64)
     return fail(ST3D_ERR_UNSUPPORTED, "the TMA kernel serves FP32 and 16-bit storage");
   if (o->kernel == ST3D_KERNEL_TMA && o->points == 2)
     return fail(ST3D_ERR_UNSUPPORTED, "the TMA kernel serves the 7/13/25-point stencils");
-  if (s16 && o->tile_j != 0 && o->tile_j != 16 &&
+  if (s16 && !mma && o->tile_j != 0 && o->tile_j != 16 &&
       !((o->tile_j == 8 || o->tile_j == 20) && o->storage != ST3D_F16_HILO))
     return fail(ST3D_ERR_UNSUPPORTED,
                 "16-bit storage runs 16-row tiles (8 or 20 also in the delta forms), not %d", o->tile_j);
@@ -602,19 +618,6 @@ int plan_tma16(st3d_ctx* c, int sm_count, int max_smem) {
   return ST3D_OK;
 }
 
-// The tensor-core kernel serves a delta-form request when asked for, or under
-// ST3D_KERNEL_AUTO when the request names no tile height or pipeline depth of
-// the scalar kernel: measured at 1024^3 on a GB300 it is the faster kernel
-// of the delta forms (25 points FP16 515 against 317 Gpts/s, BF16 498 / 312,
-// F16_HL 397 / 283; 13 points (1040^3) FP16 500 / 408, F16_HL 410 / 363;
-// 7 points FP16 615 / 545, BF16 603 / 531, F16_HL 418 / 357).
-bool mma_chosen(const st3d_opts& o) {
-  const bool delta = o.storage == ST3D_F16 || o.storage == ST3D_BF16 || o.storage == ST3D_F16_HL;
-  if (!delta || o.mode != ST3D_MODE_WAVE) return false;
-  if (o.kernel == ST3D_KERNEL_MMA) return true;
-  return o.kernel == ST3D_KERNEL_AUTO && o.tile_j == 0 && o.stages == 0;
-}
-
 // One step of a tile's plane takes this long (microseconds, all CTAs busy;
 // measured at 1024^3 and 512^3): the TALL tile's 16 warps are four a scheduler
 // (the WIDE tile's 19 five on three of them), and its store warp takes the
@@ -629,7 +632,8 @@ double mma_step_us(bool tall, int points, bool pair) {
 // Tensor-core delta-form plan (st3d_kernels_mma16.cu): the tile (MmaTile,
 // st3d_tma.cuh) with the shorter estimated step, which weighs how well it
 // fills the rows (multiples of 152 or 64 columns, 16 or 32 rows) against the
-// time above; WIDE where the request names a tile height or depth.  Measured,
+// time above; the tile of the height that the request names, WIDE where it
+// names a depth alone.  Measured,
 // us a step WIDE and TALL: FP16 25 points 512^3 326 / 290 (492 tile steps either
 // way; 1024^3, 3096 against 3672, stays WIDE: 2085), 7 points 512^3 272 / 234,
 // 1024^3 1785 / 1720; F16_HL 25 points 512^3 396 / 324, 1024^3 2710 / 2425 to
@@ -644,9 +648,10 @@ int plan_mma16(st3d_ctx* c, int sm_count, int max_smem) {
   p->pair = c->pair;
   p->mma = true;
   p->nb = 1;
-  const bool named = c->opts.tile_j > 0 || c->opts.stages > 0;
+  const bool tall_named = c->opts.tile_j == MmaTile<true>::TJ;
+  const bool wide_named = !tall_named && (c->opts.tile_j > 0 || c->opts.stages > 0);
   double best = 1e300;
-  for (int tall = 0; tall < (named ? 1 : 2); ++tall) {
+  for (int tall = tall_named ? 1 : 0; tall < (wide_named ? 1 : 2); ++tall) {
     Tma16Plan q = *p;
     q.tall = tall != 0;
     q.tj = tall ? MmaTile<true>::TJ : MmaTile<false>::TJ;
@@ -1656,10 +1661,11 @@ int st3d_plan(const st3d_grid_desc* grid, const st3d_opts* opts, st3d_info* info
   info->kernel = tma ? ST3D_KERNEL_TMA : ST3D_KERNEL_SIMPLE;
   info->tile_j = tma ? tj : 0;
   info->tile_k = tma ? kTmaTK : 0;
-  if (delta && mma_chosen(*opts)) {
+  if (mma_chosen(*opts)) {
+    const bool tall = opts->tile_j == MmaTile<true>::TJ;
     info->kernel = ST3D_KERNEL_MMA;
-    info->tile_j = 16;
-    info->tile_k = kMmaTK;
+    info->tile_j = tall ? MmaTile<true>::TJ : MmaTile<false>::TJ;
+    info->tile_k = tall ? MmaTile<true>::TK : MmaTile<false>::TK;
   }
   info->ichunk = opts->ichunk > 0 ? opts->ichunk : (tma ? 128 : 64);
   info->temporal_block = opts->temporal_block > 0 ? opts->temporal_block : 1;
