@@ -1815,7 +1815,6 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
 
   // kernel choice
   if (!c->f16) c->kernel = ST3D_KERNEL_SIMPLE;
-  c->ichunk = c->opts.ichunk > 0 ? c->opts.ichunk : 64;
   if (c->opts.storage == ST3D_F32 && c->opts.points != 2 && c->opts.kernel != ST3D_KERNEL_SIMPLE) {
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
@@ -1842,6 +1841,9 @@ int st3d::create_context(const st3d_grid_desc* grid, const st3d_opts* opts, cuda
                             "the TMA kernel cannot run with this configuration"));
     }
   }
+  if (c->kernel == ST3D_KERNEL_SIMPLE)
+    c->ichunk = c->opts.ichunk > 0 ? c->opts.ichunk
+                                   : simple_ichunk(c->opts.points, c->opts.mode, c->opts.storage, c->G);
   // (options that name a tile height, unit length or pipeline depth ask for
   // the one-step kernel in that shape)
   if (c->opts.tile_j <= 0 && c->opts.ichunk <= 0 && c->opts.stages <= 0) setup_wave(c, sm);
@@ -2131,7 +2133,7 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     } else {
       const void* cf = c->opts.storage == ST3D_F64 ? (const void*)&c->cf64 : (const void*)&c->cf32;
       e = launch_simple(c->opts.points, c->opts.mode, c->opts.storage, c->G, cf, v_ptr(c),
-                        u_ptr(c), c->fld[2], src, c->opts.ichunk, (int)take, c->stream);
+                        u_ptr(c), c->fld[2], src, c->ichunk, (int)take, c->stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "stencil kernel launch");
     ++c->launches;

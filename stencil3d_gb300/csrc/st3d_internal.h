@@ -188,6 +188,8 @@ constexpr int kRefSteps = 1024;
 cudaError_t launch_simple(int points, int mode, int storage, const Geom& g, const void* coefs,
                           void* v, const void* u, const void* s, const Source& src,
                           int ichunk, int rsteps, cudaStream_t stream);
+// Planes per block of the direct-load kernel where the request names none (current device).
+int simple_ichunk(int points, int mode, int storage, const Geom& g);
 
 struct TmaPlan;
 // ubuf/vbuf/sbuf select the tensor maps of the field buffers holding u, v, s.

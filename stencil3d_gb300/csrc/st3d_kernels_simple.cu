@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Planes per block where the caller names none (ichunk 0): the chunk whose
+// Planes per block where the caller names none: the chunk whose
 // blocks fill the GPU's last round best, each with its 2R planes of queue to
 // load first (about a tenth of a plane's time each).  FP64, 25 points, 256^3:
 // 64 planes make 1.7 rounds of blocks, 853 us a step; 37 planes 2.9 rounds,
@@ -237,27 +237,44 @@ int pick_chunk(long long columns, int xs, int slots, int R) {
 }
 
 template <typename T, int P, int MODE>
+int chunk_t(const Geom& g) {
+  if constexpr (P == 2) {
+    return 64;
+  } else {
+    int per_sm = 0, dev = 0, sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_simple<T, P, MODE>, kSimpleBX * kSimpleBY, 0) !=
+            cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      return 64;
+    }
+    if (sm * per_sm < 1) return 64;
+    return pick_chunk((long long)((g.zs + kSimpleBX - 1) / kSimpleBX) * ((g.ys + kSimpleBY - 1) / kSimpleBY),
+                      g.xs, sm * per_sm, P == 25 ? 4 : P == 13 ? 2 : 1);
+  }
+}
+
+template <typename T>
+int chunk_typed(int points, int mode, const Geom& g) {
+#define ST3D_CASE(PTS)                                                                      \
+  case PTS:                                                                                 \
+    return mode == ST3D_MODE_REF ? chunk_t<T, PTS, ST3D_MODE_REF>(g) : chunk_t<T, PTS, ST3D_MODE_WAVE>(g);
+  switch (points) {
+    ST3D_CASE(7)
+    ST3D_CASE(13)
+    ST3D_CASE(25)
+    default:
+      return 64;
+  }
+#undef ST3D_CASE
+}
+
+template <typename T, int P, int MODE>
 cudaError_t launch_t(const Geom& g, const void* coefs, void* v, const void* u, const void* s,
                      const Source& src, int ichunk, int rsteps, cudaStream_t stream) {
   const Coefs<T>& cf = *static_cast<const Coefs<T>*>(coefs);
   dim3 block(kSimpleBX, kSimpleBY, 1);
-  if (ichunk <= 0) {
-    ichunk = 64;
-    if constexpr (P != 2) {
-      static const int per_sm = [] {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_simple<T, P, MODE>, kSimpleBX * kSimpleBY, 0) !=
-            cudaSuccess)
-          cudaGetLastError();
-        return n;
-      }();
-      int dev = 0, sm = 0;
-      if (cudaGetDevice(&dev) == cudaSuccess &&
-          cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sm * per_sm > 0)
-        ichunk = pick_chunk((long long)((g.zs + kSimpleBX - 1) / kSimpleBX) * ((g.ys + kSimpleBY - 1) / kSimpleBY),
-                            g.xs, sm * per_sm, P == 25 ? 4 : P == 13 ? 2 : 1);
-    }
-  }
   dim3 grid((g.zs + kSimpleBX - 1) / kSimpleBX, (g.ys + kSimpleBY - 1) / kSimpleBY,
             (g.xs + ichunk - 1) / ichunk);
   if constexpr (P == 2) {
@@ -301,6 +318,10 @@ cudaError_t launch_typed(int points, int mode, const Geom& g, const void* coefs,
 }
 
 }  // namespace
+
+int simple_ichunk(int points, int mode, int storage, const Geom& g) {
+  return storage == ST3D_F64 ? chunk_typed<double>(points, mode, g) : chunk_typed<float>(points, mode, g);
+}
 
 cudaError_t launch_simple(int points, int mode, int storage, const Geom& g, const void* coefs,
                           void* v, const void* u, const void* s, const Source& src, int ichunk,
