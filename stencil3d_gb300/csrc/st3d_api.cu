@@ -1028,25 +1028,25 @@ double single_step_us(const st3d_ctx* c) {
 
 // Lays T levels of the tile shape `nar` out on `ctas` CTAs; false where the
 // columns or levels are more than the progress words hold.
-bool wave_layout(WavePlan* w, int nar, int T, int ctas, const Layout& L, int R) {
-  const WaveShape& sh = w->shape[nar];
-  w->narrow = nar;
-  w->T = T;
-  w->skew = w->shift = 0;
-  w->Q = sh.ntj * sh.ntk;
-  if (w->Q > ctas / T) {
+bool wave_layout(const WavePlan& w, int nar, int T, int ctas, const Layout& L, int R, WaveLayout* v) {
+  const WaveShape& sh = w.shape[nar];
+  v->narrow = nar;
+  v->T = T;
+  v->skew = v->shift = 0;
+  v->Q = sh.ntj * sh.ntk;
+  if (v->Q > ctas / T) {
     // several turns: each level R rows lower and one column later
-    w->skew = R;
-    w->shift = 1;
-    w->Q = (int)(((long long)L.ys + (T - 1) * R + sh.tj - 1) / sh.tj) * sh.ntk;
+    v->skew = R;
+    v->shift = 1;
+    v->Q = (int)(((long long)L.ys + (T - 1) * R + sh.tj - 1) / sh.tj) * sh.ntk;
   }
-  w->S = std::min(w->Q, ctas / T);
-  return T <= kWaveLevels && w->S >= 1 && w->Q <= w->max_columns;
+  v->S = std::min(v->Q, ctas / T);
+  return T <= kWaveLevels && v->S >= 1 && v->Q <= w.max_columns;
 }
 // Columns one CTA takes one after the other for n steps.
-double wave_turns(const WavePlan& w, int n) {
-  const long long passes = (n + w.T - 1) / w.T;
-  return (double)((passes * w.Q + (long long)(w.T - 1) * w.shift + w.S - 1) / w.S);
+double wave_turns(const WaveLayout& v, int n) {
+  const long long passes = (n + v.T - 1) / v.T;
+  return (double)((passes * v.Q + (long long)(v.T - 1) * v.shift + v.S - 1) / v.S);
 }
 
 // The shape of a launch of `steps` wave steps; false: one step a launch is
@@ -1080,22 +1080,25 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
   static const double levels[7] = {0.0, 0.0, 1.08, 1.05, 1.0, 1.0, 1.18};
   double best = 1e300;
   int best_T = 0;
+  WaveLayout taken;
   for (int nar = 0; nar < 2; ++nar) {
     for (int T = 2; T <= std::min({n, c->wave->ctas, 24}); ++T) {
-      WavePlan v = *c->wave;
-      if (!wave_layout(&v, nar, T, v.ctas, c->L, R)) break;
+      WaveLayout v;
+      if (!wave_layout(*c->wave, nar, T, c->wave->ctas, c->L, R, &v)) break;
       const double us = wave_turns(v, n) * (xs + 2.0 * R) * tau * (nar ? 1.05 : 1.0) *
                             (size == 2 ? levels[std::min(T, 6)] : !v.shift ? 1.0 : T > 5 ? 1.3 : 1.15) +
                         (6.0 + R) * (T - 1) + 12.0;
       if (us < best) {
         best = us;
         best_T = T;
-        *w = v;
+        taken = v;
       }
     }
   }
   if (!best_T || (!any && best > 0.93 * n * single_step_us(c))) return false;
   if (est_us) *est_us = best;
+  *w = *c->wave;
+  static_cast<WaveLayout&>(*w) = taken;
   // beyond R + 1 planes, or the slowest of two neighbours could wait for the
   // other (16 / 20 / 26 / 32 planes, Gpts/s: 25 points, 1024^2 planes 439 / 467 /
   // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497); unbounded (7 points 256^3, 201 MB: 590 against 618 us) where L2
@@ -1129,12 +1132,12 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
   const int ctas = w.ctas - x.n_up - x.n_down;
   double best = 1e300;
   for (int nar = 0; nar < 2; ++nar) {
-    WavePlan v = w;
-    if (!wave_layout(&v, nar, n, ctas, c->L, R)) continue;
+    WaveLayout v;
+    if (!wave_layout(w, nar, n, ctas, c->L, R, &v)) continue;
     const double us = wave_turns(v, n) * (xs + 2 * R) * (nar ? 1.05 : 1.0);
     if (us < best) {
       best = us;
-      w = v;
+      static_cast<WaveLayout&>(w) = v;
     }
   }
   if (best > 1e299) return ST3D_OK;
@@ -2030,6 +2033,7 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     ++c->launches;
     iterations -= T;
   }
+  uint32_t declined = 0;  // a number of steps that one launch is not the choice for
   for (uint32_t n = 0; n < iterations;) {
     // FP32 wave: many steps a launch, from shared memory where the grid fits
     // (any run of 3 steps is faster there: 7 points 64^3 15.0 us against 22.7,
@@ -2040,7 +2044,9 @@ int st3d_iterate(st3d_ctx* c, uint32_t iterations) {
     const uint32_t many = brick     ? std::min(left, (uint32_t)kWaveSteps)
                           : c->wave ? std::min(left, (uint32_t)c->wave->max_steps)
                                     : 0u;
-    if (brick || plan_wave(c, many, &wp)) {
+    const bool planned = !brick && many != declined && plan_wave(c, many, &wp);
+    if (!planned) declined = many;
+    if (brick || planned) {
       Source src;
       src.i = c->opts.src_i; src.j = c->opts.src_j; src.k = c->opts.src_k;
       src.amp = 0.0f; src.amp_d = 0.0;

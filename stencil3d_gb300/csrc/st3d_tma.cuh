@@ -127,16 +127,18 @@ struct WaveShape {
   CUtensorMap umap[2];       // halo box over the u/v pair
   CUtensorMap vmap[3];       // interior box over the pair and s
 };
-struct WavePlan {
-  WaveShape shape[2];        // 16 x 128 and 32 x 64 tiles
-  int ctas = 0;              // CTAs the GPU holds at once
-  int max_steps = 0;         // steps the words are enough for
-  int max_columns = 0;       // and columns
+struct WaveLayout {
   int narrow = 0;            // the shape taken
   int T = 1, S = 1;          // levels, columns at work in each
   int Q = 0;                 // columns: the tiles of all levels' rows
   int shift = 0;             // columns a level starts behind the one before
   int skew = 0;              // rows a tile lies lower at each level
+};
+struct WavePlan : WaveLayout {
+  WaveShape shape[2];        // 16 x 128 and 32 x 64 tiles
+  int ctas = 0;              // CTAs the GPU holds at once
+  int max_steps = 0;         // steps the words are enough for
+  int max_columns = 0;       // and columns
   int couple = 0;            // planes a column of level 0 may be ahead of its neighbours
   int* words = nullptr;      // progress words (device)
   size_t words_n = 0;
