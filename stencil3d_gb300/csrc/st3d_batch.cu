@@ -444,6 +444,7 @@ struct st3d_batch {
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     int2* items = nullptr;  // the queue of the grids that step together (device)
+    uint64_t launches = 0;  // kernel launches captured
   };
   std::map<uint32_t, Graph> graphs;  // by step count
   int device = -1;  // CUDA device ordinal of every grid (opts.device), -1: current
@@ -611,7 +612,7 @@ std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
 
 // The multi-step launches of the grids that run alone, u's buffer and the
 // amplitudes read from device memory (the launches are captured).
-int enqueue_alone(st3d_batch* b, uint32_t steps, const std::vector<char>& alone) {
+cudaError_t enqueue_alone(st3d_batch* b, uint32_t steps, const std::vector<char>& alone, uint64_t* launches) {
   const int n = (int)b->ctx.size();
   for (int gi = 0; gi < n; ++gi) {
     if (!alone[gi]) continue;
@@ -628,23 +629,28 @@ int enqueue_alone(st3d_batch* b, uint32_t steps, const std::vector<char>& alone)
       feed.ub_dev = &b->d_grids[gi].cur0;
       feed.amps_dev = b->d_amps + (size_t)done * n + gi;
       feed.amp_stride = n;
+      cudaError_t e;
       if (brick) {
-        B_CUDA(launch_brick(c->brick, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed,
-                            c->brick_words, c->dev_status, b->stream));
+        e = launch_brick(c->brick, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed, c->brick_words,
+                         c->dev_status, b->stream);
       } else {
         WavePlan w;
-        if (!plan_wave(c, many, &w, nullptr, true)) return bfail(ST3D_ERR_CUDA, "no multi-step launch");
-        B_CUDA(launch_wave(w, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed, c->dev_status,
-                           b->stream));
+        e = !plan_wave(c, many, &w, nullptr, true)
+                ? cudaErrorCooperativeLaunchTooLarge
+                : launch_wave(w, c->opts.points, c->G, c->cf32, fld, (int)many, src, feed, c->dev_status, b->stream);
       }
+      if (e != cudaSuccess) return e;
+      ++*launches;
       done += many;
     }
   }
-  return ST3D_OK;
+  return cudaSuccess;
 }
 
-// Captures one call of `steps` steps.
-int capture_graph(st3d_batch* b, uint32_t steps, const std::vector<char>& alone, st3d_batch::Graph* out) {
+// Captures one call of `steps` steps.  *too_large: the failure is that the GPU
+// cannot hold a multi-step launch of the grids that run alone.
+int capture_graph(st3d_batch* b, uint32_t steps, const std::vector<char>& alone, st3d_batch::Graph* out,
+                  bool* too_large) {
   std::vector<int2> items;
   for (const int2& it : b->items)
     if (!alone[it.x]) items.push_back(it);
@@ -656,13 +662,21 @@ int capture_graph(st3d_batch* b, uint32_t steps, const std::vector<char>& alone,
   }
   cudaGraph_t graph = nullptr;
   B_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_alone(b, steps, alone);
-  if (rc == ST3D_OK && !items.empty()) rc = enqueue_persistent(b, steps, out->items, (int)items.size());
-  cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+  out->launches = 0;
+  cudaError_t e = enqueue_alone(b, steps, alone, &out->launches);
+  *too_large = e == cudaErrorCooperativeLaunchTooLarge;
+  int rc = e == cudaSuccess ? ST3D_OK
+                            : set_error(ST3D_ERR_CUDA, "multi-step launch of a batch's grid: %s", cudaGetErrorString(e));
+  if (rc == ST3D_OK && !items.empty()) {
+    rc = enqueue_persistent(b, steps, out->items, (int)items.size());
+    out->launches += steps;
+  }
+  e = cudaStreamEndCapture(b->stream, &graph);
   if (rc == ST3D_OK && e != cudaSuccess)
     rc = set_error(ST3D_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
   if (rc == ST3D_OK) {
     e = cudaGraphInstantiate(&out->exec, graph, 0);
+    *too_large = e == cudaErrorCooperativeLaunchTooLarge;
     if (e != cudaSuccess) rc = set_error(ST3D_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
   }
   if (graph) cudaGraphDestroy(graph);
@@ -918,20 +932,22 @@ int st3d_batch_iterate(st3d_batch* b, uint32_t steps, int schedule) {
   }
   if (schedule == ST3D_BATCH_PERSISTENT) {
     if ((rc = enqueue_persistent(b, steps, b->d_items, b->total_items)) != ST3D_OK) return rc;
+    b->launches += steps;
   } else {
     auto it = b->graphs.find(steps);
     if (it == b->graphs.end()) {
       st3d_batch::Graph graph;
       const std::vector<char> none(b->ctx.size(), 0), alone = split_grids(b, steps);
-      rc = capture_graph(b, steps, alone, &graph);
+      bool too_large = false;
+      rc = capture_graph(b, steps, alone, &graph, &too_large);
       // a GPU that cannot hold a multi-step launch: every grid in the queue
-      if (rc != ST3D_OK && alone != none) rc = capture_graph(b, steps, none, &graph);
+      if (rc != ST3D_OK && too_large) rc = capture_graph(b, steps, none, &graph, &too_large);
       if (rc != ST3D_OK) return rc;
       it = b->graphs.emplace(steps, graph).first;
     }
     B_CUDA(cudaGraphLaunch(it->second.exec, b->stream));
+    b->launches += it->second.launches;
   }
-  b->launches += steps;
   advance(b, steps);
   return ST3D_OK;
 }
