@@ -1014,7 +1014,8 @@ void setup_wave(st3d_ctx* c, int sm_count) {
     delete w;
     return;
   }
-  c->wave = w;  // its words, like the other scratch, are not counted in c->bytes
+  c->wave = w;
+  c->bytes += w->words_n * sizeof(int);
 }
 
 // Estimated time of one step a launch (see plan_wave).
