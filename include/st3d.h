@@ -182,7 +182,10 @@ typedef struct st3d_info {
   int32_t host_path;          /* st3d_host_path of the last upload or download */
   int32_t tb_tile_j;          /* rows of a temporally blocked pass's level-1 tile; 0 = none */
   int32_t device;             /* CUDA device ordinal of the context (st3d_plan: opts.device) */
-  int32_t reserved[5];
+  /* the last streamed call: levels of its pipeline over rows of tiles and the
+   * rows of a tile (16 or 32); 0: it ran over chunks of planes, or there was none */
+  int32_t stream_levels, stream_tile_j;
+  int32_t reserved[3];
 } st3d_info;
 
 typedef struct st3d_ctx st3d_ctx;

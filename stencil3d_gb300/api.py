@@ -62,7 +62,8 @@ class Info(C.Structure):
                 ("bytes_per_point", C.c_double), ("flops_per_point", C.c_double),
                 ("tile_j", C.c_int32), ("tile_k", C.c_int32), ("ichunk", C.c_int32),
                 ("temporal_block", C.c_int32), ("host_path", C.c_int32), ("tb_tile_j", C.c_int32),
-                ("device", C.c_int32), ("reserved", C.c_int32 * 5)]
+                ("device", C.c_int32), ("stream_levels", C.c_int32), ("stream_tile_j", C.c_int32),
+                ("reserved", C.c_int32 * 3)]
 
 
 class Metrics(C.Structure):

@@ -1184,6 +1184,8 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
   c->launches += 1;
   if (n & 1) std::swap(c->ub, c->vb);
   c->host_path = ST3D_HOST_STREAMED;
+  c->stream_levels = w.T;
+  c->stream_tile_j = w.shape[w.narrow].tj;
   *done = true;
   return ST3D_OK;
 }
@@ -1407,6 +1409,7 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
     c->vb = t;
   }
   c->host_path = ST3D_HOST_STREAMED;
+  c->stream_levels = c->stream_tile_j = 0;
   *done = true;
   return ST3D_OK;
 }
@@ -1908,6 +1911,8 @@ int st3d_get_info(const st3d_ctx* c, st3d_info* info) {
   info->host_path = c->host_path;
   info->tb_tile_j = c->tb ? c->tb->rows : 0;
   info->device = c->device;
+  info->stream_levels = c->stream_levels;
+  info->stream_tile_j = c->stream_tile_j;
   return ST3D_OK;
 }
 

@@ -77,6 +77,8 @@ struct st3d_ctx {
   // the same for grids that fit the SMs' shared memory (st3d_kernels_brick.cu)
   st3d::BrickPlan brick;  // nbi = 0: none
   int* brick_words = nullptr;  // part of `scratch`
+  // the last streamed call: levels and rows of a tile on the multi-step kernel; 0: chunks
+  int stream_levels = 0, stream_tile_j = 0;
   // the streamed drop-in call (st3d_stream.cu): its queues, counters and
   // amplitudes on the device, and their host copies (kept until the next call)
   void* stream_buf = nullptr;
