@@ -1058,16 +1058,18 @@ double wave_turns(const WaveLayout& v, int n) {
 //     up to 300 MB and 0.55 / 0.56 / 0.62 beyond, where 4 and 5 levels are best
 //     (Gpts/s with 2 / 3 / 4 / 5 / 6 levels: 7 points, 1024^2 planes 484 / 518 /
 //     571 / 589 / 516; 25 points 443 / 434 / 463 / 463 / 381);
-//     several turns below 300 MB 15 % more (13 points 301 x 187 x 423: 48
-//     columns at once in 3 levels 1058 us, 38 at a time in 4 levels 1160),
-//     30 % with more than 5 levels;
+//     several turns below 300 MB 15 % more, 30 % with more than 5 levels (20
+//     steps in 3 / 4 / 5 / 6 levels, us: 7 points 272^3 909 / 840 / 776 / 969, 288^3
+//     986 / 964 / 946 / 1042, 200 x 400 x 260 974 / 877 / 854 / 991; 13 points 272^3
+//     974 / 903 / 834 / 1051, 301 x 187 x 423 1083 / 1061 / 1090 / 1304; all levels of
+//     3 are one turn);
 //     a level starts 6 + R us after the one before; 32 x 64 tiles take 5 % more
 //     a plane and pay off where they pad less (25 points 528^3: 420 against
 //     380 Gpts/s);
 //   one step a launch: its units' planes (with R warm-up planes) at 0.76 us
 //     where the tiles are full (padding costs no HBM bytes), 0.5 in L2, and
 //     3.5 us a launch.
-// Measured (one step a launch -> several): 7 points 256^3 x 20 937 -> 590 us,
+// Measured (one step a launch -> several): 7 points 256^3 x 20 937 -> 665 us,
 // 13 points 301 x 187 x 423 x 20 1413 -> 1058, 25 points 528^3 x 40 15969 ->
 // 14009, 1024^3 x 20 54748 -> 45771; 7 points 128^3 x 20 stays at one (145
 // against 159).
@@ -1102,8 +1104,14 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
   static_cast<WaveLayout&>(*w) = taken;
   // beyond R + 1 planes, or the slowest of two neighbours could wait for the
   // other (16 / 20 / 26 / 32 planes, Gpts/s: 25 points, 1024^2 planes 439 / 467 /
-  // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497); unbounded (7 points 256^3, 201 MB: 590 against 618 us) where L2
-  // has room (13 points 301 x 187 x 423, 286 MB: 1149 against 1044)
+  // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497).  Above 240 MB coupling gains
+  // at 7 and 13 points (20 steps, free -> coupled, us: 7 points 272^3 865 -> 839, 288^3
+  // 1046 -> 986, 320^3 1494 -> 1225, 400 x 180 x 300 910 -> 788) and costs 25 points 1 %
+  // at most up to 300 MB.  Below 120 MB, where L2 holds the fields, it costs up to 5 %
+  // (200^3 363 -> 379).  Between the two it goes either way: 240^3 526 -> 479, 256^3
+  // 665 -> 620, 128 x 384 x 384 858 -> 775, but 600 x 160 x 200 764 -> 798, 500 x 128 x
+  // 256 624 -> 676, 420 x 140 x 260 692 -> 751 (long calls gain more, 60 steps 256^3 13 %);
+  // no size alone tells them apart, so these run free.
   w->couple = bytes > 2.4e8 ? kWaveCouple : 1 << 28;
   w->limit_ns = 4000000000ull + (uint64_t)(bytes / 12.0 * n / 2.5);
   return true;
