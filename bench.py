@@ -185,6 +185,37 @@ def profile_traffic(kernel_tag, workload):
     return None
 
 
+def multi_step_bytes(workload):
+    """HBM bytes per point and step of a launch of many wave steps, as the
+    committed ncu summary of the order and plane size counted them
+    (profiles/wave_<points>_<edge>.md, line 'traffic_bytes_per_point_step:');
+    None without one."""
+    points, _, ys, zs = WORKLOADS[workload][:4]
+    try:
+        for line in open(os.path.join(REPO, "profiles", "wave_%d_%d.md" % (points, zs if ys == zs else 0))):
+            if line.startswith("traffic_bytes_per_point_step:"):
+                return float(line.split(":", 1)[1].split()[0])
+    except OSError:
+        pass
+    return None
+
+
+def wave_roofline(info, workload, pts, steps, ms, launches, peak):
+    """HBM roofline of FP32 wave steps.  A launch of one step (or of one fused
+    pass) moves the algorithmic bytes.  Planes of a launch of many steps meet
+    in L2: its bytes are the profiled ones, and `one_round` is the rate that
+    the algorithmic bytes of every step would make, which may pass the peak."""
+    rate = pts * steps / (ms * 1e-3) / 1e9  # Gpts/s
+    out = {"achieved": info.bytes_per_point * rate, "peak": peak, "unit": "GB/s",
+           "bytes_per_point": info.bytes_per_point}
+    if info.temporal_block <= 1 and launches < steps:
+        out["one_round"] = {"gbs": out["achieved"], "frac": out["achieved"] / peak}
+        out["bytes_per_point"] = multi_step_bytes(workload)
+        out["achieved"] = out["bytes_per_point"] and out["bytes_per_point"] * rate
+    out["frac"] = out["achieved"] and out["achieved"] / peak
+    return out
+
+
 # --------------------------------------------------------------------------
 def make_stencil(S, wl, storage="f32", kernel="auto", temporal_block=1, **kw):
     kw.setdefault("device", DEVICE)
@@ -369,13 +400,11 @@ def temporal_run(S, workloads, steps, warmup, peak):
             st.synchronize()
             launches = st.info().launches - l0
             pts = g.gvol
-            ach = info.bytes_per_point * pts * n / (ms * 1e-3) / 1e9
             entry = {"value": pts * n / (ms * 1e-3) / 1e9, "unit": "Gpts/s",
                      "ms_per_step": ms / n, "launches": int(launches),
                      "bytes_per_point_step": info.bytes_per_point,
                      "tile_rows": int(info.tb_tile_j or info.tile_j),
-                     "roofline": {"achieved": ach, "peak": peak, "unit": "GB/s",
-                                  "frac": ach / peak}}
+                     "roofline": wave_roofline(info, wl, pts, n, ms, launches, peak)}
             if ref is None:
                 ref = st
             else:
@@ -435,16 +464,17 @@ def config_runs(S, warmup, peak):
             info = st.info()
             st.iterate(warmup)
             st.synchronize()
+            l0 = st.info().launches
             st.timer_start()
             st.iterate(steps)
             ms = st.timer_stop()
             st.synchronize()
+            launches = st.info().launches - l0
         finally:
             st.close()
-        ach = info.bytes_per_point * g.gvol * steps / (ms * 1e-3) / 1e9
         out[wl] = {"value": g.gvol * steps / (ms * 1e-3) / 1e9, "unit": "Gpts/s", "steps": steps,
                    "ms_per_step": ms / steps, "fields_gb": round(3 * g.gsize * 4 / 1e9, 3),
-                   "roofline": {"achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak}}
+                   "roofline": wave_roofline(info, wl, g.gvol, steps, ms, launches, peak)}
     return out
 
 
@@ -610,12 +640,15 @@ def run_gb300(args, dist):
     pts = g.gvol
     value = dist.world * pts * args.steps / (ms_max * 1e-3) / 1e9
     peak, peak_kind = measured_peak()
-    # algorithmic bytes of every step over the timed region; a launch of
-    # several steps meets part of them in L2, so the rate may pass the HBM peak
-    achieved = info.bytes_per_point * pts * args.steps / (ms * 1e-3) / 1e9
     kernel_tag = "tma" if info.kernel == S.KERNEL_TMA else "simple"
     many = launches < args.steps
-    traffic = None if many else profile_traffic(kernel_tag, args.workload)
+    roofline = wave_roofline(info, args.workload, pts, args.steps, ms, launches, peak)
+    roofline.update(
+        bound="hbm", peak_kind=peak_kind,
+        traffic=(roofline["bytes_per_point"] and roofline["bytes_per_point"] * pts * args.steps / launches)
+        if many else profile_traffic(kernel_tag, args.workload),
+        kernel="k_wave<%d>" % points if many else
+        "k_tma<%d,wave>" % points if kernel_tag == "tma" else "k_simple<float,%d,wave>" % points)
 
     result = {
         "metric": "Gpts/s + % of HBM roofline, 25-pt 1024^3: FP32 vs FP16-store at stated L2 err",
@@ -630,13 +663,7 @@ def run_gb300(args, dist):
                    "l2": l2_note(info),
                    "parallelism": "replicas" if dist.world > 1 else "single GPU"},
         "gflops": pts * args.steps * info.flops_per_point / (ms * 1e-3) / 1e9,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "peak_kind": peak_kind,
-                     "bytes_per_point": info.bytes_per_point,
-                     "traffic": traffic,
-                     "kernel": "k_wave<%d>" % points if many else
-                               "k_tma<%d,wave>" % points if kernel_tag == "tma" else
-                               "k_simple<float,%d,wave>" % points},
+        "roofline": roofline,
         "gpu_launches": int(launches),
         "clocks": clk,
         "fp16": None,
@@ -666,11 +693,12 @@ def run_gb300(args, dist):
         # the plain kernel in FP64, 32 algorithmic bytes per point
         gp, msd, dinfo = time_storage(S, args.workload, "f64", args.fp64_steps, min(args.warmup, 3))
         ach = dinfo.bytes_per_point * pts / (msd * 1e-3) / 1e9
-        # FP64 arithmetic per point of the wave update: 3 per neighbour pair
-        # ((a+b), -2u, fma) plus 2u, -v and two fma; each one FP64-pipe
-        # instruction, against the nominal 1.25 TFLOP/s = 0.625 T FP64 fma/s
+        # FP64-pipe instructions per point of the wave update: one multiply-add
+        # per neighbour pair, 2u - v and two more (the pairs' sums run as
+        # integers where their exponents allow), against the nominal
+        # 1.25 TFLOP/s = 0.625 T FP64 fma/s
         npairs = {7: 3, 13: 6, 25: 12}[points]
-        dp_ops = 3 * npairs + 4
+        dp_ops = npairs + 3
         dp_rate = dp_ops * pts / (msd * 1e-3) / 1e12
         result["fp64"] = {"value": dist.world * gp * (ms / ms_max), "unit": "Gpts/s",
                           "ms_per_step": msd, "bytes_per_point": dinfo.bytes_per_point,
