@@ -74,12 +74,13 @@ ST3D_HD uint64_t add_scaled(uint64_t acc, uint32_t hi, uint32_t lo, uint32_t p, 
 }
 
 constexpr uint32_t kExpMask = 0x7ff00000u;  // exponents stay where they are, in bits 20..30
-constexpr int kExpOne = 1 << 20;
-constexpr int kGuard = 8;  // 3 * 2^(53 + kGuard) < 2^63
+constexpr uint32_t kExpOne = 1u << 20;
+constexpr uint32_t kExpInfinite = 2047u * kExpOne;
+constexpr uint32_t kGuard = 8;  // 3 * 2^(53 + kGuard) < 2^63
 
 // The centre's -2u as the sums take it.
 struct Twice {
-  int e;             // exponent bits of 2u
+  uint32_t e;        // exponent bits of 2u, kExpInfinite and above where 2u is not finite
   uint32_t hi, lo;   // significand with its leading bit
   uint32_t neg;      // all ones where -2u is negative
 };
@@ -88,8 +89,7 @@ ST3D_HD Twice twice_of(double u) {
   const Bits64 b = bits_of(u);
   Twice t;
   const uint32_t e = b.hi & kExpMask;
-  // 0, which fails the range check, for zero and subnormal u and where 2u is not finite
-  t.e = e - kExpOne < 2045u * kExpOne ? (int)(e + kExpOne) : 0;
+  t.e = e ? e + kExpOne : 0u;  // zero and subnormal u fail the range check
   t.hi = (b.hi & 0xfffffu) | 0x100000u;
   t.lo = b.lo;
   t.neg = ~(uint32_t)((int32_t)b.hi >> 31);
@@ -97,22 +97,22 @@ ST3D_HD Twice twice_of(double u) {
 }
 
 // Whether the integer path serves this pair; the exponents' top in *E.
-ST3D_HD bool pair_fits(const Bits64& a, const Bits64& b, const Twice& u, int* E) {
-  const int ea = (int)(a.hi & kExpMask), eb = (int)(b.hi & kExpMask);
-  const int top = ea > eb ? (ea > u.e ? ea : u.e) : (eb > u.e ? eb : u.e);
-  const int low = ea < eb ? (ea < u.e ? ea : u.e) : (eb < u.e ? eb : u.e);
+ST3D_HD bool pair_fits(const Bits64& a, const Bits64& b, const Twice& u, uint32_t* E) {
+  const uint32_t ea = a.hi & kExpMask, eb = b.hi & kExpMask;
+  const uint32_t top = ea > eb ? (ea > u.e ? ea : u.e) : (eb > u.e ? eb : u.e);
+  const uint32_t low = ea < eb ? (ea < u.e ? ea : u.e) : (eb < u.e ? eb : u.e);
   *E = top;
   // 64 <= low and top <= 2044 hold together where low lies in 64 .. 2036
-  return top - low <= kGuard * kExpOne && (uint32_t)(low - 64 * kExpOne) <= 1972u * kExpOne;
+  return top - low <= kGuard * kExpOne && low - 64u * kExpOne <= 1972u * kExpOne;
 }
 
 // rn(rn(a + b) - 2u) for operands that fit, in *d; false where the difference
 // cancels below 2^32 of its 61-bit scale and the FP64 unit has to form it.
-ST3D_HD bool pair_diff_bits(const Bits64& a, const Bits64& b, const Twice& u, int E, double* out) {
-  const int base = E - kGuard * kExpOne;
+ST3D_HD bool pair_diff_bits(const Bits64& a, const Bits64& b, const Twice& u, uint32_t E, double* out) {
+  const uint32_t base = E - kGuard * kExpOne;
   const uint32_t sa = (uint32_t)((int32_t)a.hi >> 31), sb = (uint32_t)((int32_t)b.hi >> 31);
-  const uint32_t pa = (sa | 1u) << (((int)(a.hi & kExpMask) - base) >> 20);
-  const uint32_t pb = (sb | 1u) << (((int)(b.hi & kExpMask) - base) >> 20);
+  const uint32_t pa = (sa | 1u) << (((a.hi & kExpMask) - base) >> 20);
+  const uint32_t pb = (sb | 1u) << (((b.hi & kExpMask) - base) >> 20);
   const uint32_t pu = (u.neg | 1u) << ((u.e - base) >> 20);
   uint64_t t = add_scaled(0, (a.hi & 0xfffffu) | 0x100000u, a.lo, pa, sa);
   t = add_scaled(t, (b.hi & 0xfffffu) | 0x100000u, b.lo, pb, sb);
@@ -134,7 +134,7 @@ ST3D_HD bool pair_diff_bits(const Bits64& a, const Bits64& b, const Twice& u, in
   const int z = 30 - top_bit(mh);
   uint64_t n = m * (uint64_t)(1u << (z & 31));
   n += 0x1ffu + (((uint32_t)n >> 10) & 1u);
-  const uint32_t hi = (uint32_t)(n >> 42) + (uint32_t)(E + kExpOne - z * kExpOne);
+  const uint32_t hi = (uint32_t)(n >> 42) + E + kExpOne - (uint32_t)z * kExpOne;
   *out = double_of(hi + (sd << 31), (uint32_t)(n >> 10));
   return mh != 0;
 }

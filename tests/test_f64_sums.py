@@ -27,7 +27,7 @@ static double make(uint64_t exponent) {
 static long served = 0, wrong = 0;
 static void pair(double a, double b, double u) {
   const Twice t = twice_of(u);
-  int E;
+  uint32_t E;
   double d;
   if (!pair_fits(bits_of(a), bits_of(b), t, &E)) return;
   if (!pair_diff_bits(bits_of(a), bits_of(b), t, E, &d)) return;
