@@ -129,9 +129,9 @@ typedef struct st3d_grid_desc {
  * as it is done; the same bits as the phase-by-phase call.  AUTO takes it for
  * FP32 contexts on the TMA kernel's default tiles without temporal blocking
  * when v, s and u are pinned, except for mode W calls of more than 32 steps
- * that are estimated to run faster phase by phase: small grids, and large ones
- * from some 40 (512^3) to 70 (1024^3) steps on (asking for STREAMED where it
- * does not apply runs DIRECT). */
+ * that are estimated to run faster phase by phase: small and thin grids, and
+ * others from some 40 (512^3) to 70 (1024^3) steps on (asking for STREAMED where
+ * it does not apply runs DIRECT). */
 typedef enum st3d_host_path {
   ST3D_HOST_AUTO = 0,
   ST3D_HOST_STAGED = 1,

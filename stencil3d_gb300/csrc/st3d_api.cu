@@ -1219,22 +1219,26 @@ double steps_us(const st3d_ctx* c, uint32_t n) {
 // Whether a wave call of more steps than the pipeline of levels takes
 // (iterate_host_wave) runs faster over chunks of planes beside its transfers
 // (st3d_stream.cu) or phase by phase, the steps many a launch with all CTAs.
-// Chunks hide the downloads and most of the uploads, but step slower: an item
-// (16 planes of a tile) takes 11 / 11.6 / 14.3 us at 7 / 13 / 25 points on about 108
-// CTAs, and a (step, chunk) waits for the one before, so fewer tiles than CTAs
-// leave CTAs idle.  Pinned arrays, ms a call in chunks / in phases: 7 points 512^3
-// 33 steps 19.5 / 21.3, 48 steps 25.7 / 24.6; 1024^3 33 steps 122 / 173, 64 steps
-// 215 / 227, 100 steps 324 / 294; 25 points 1024^3 33 steps 140 / 185, 100 steps
-// 379 / 335; 768^3 33 steps 70.4 / 77.9, 48 steps 99.2 / 91.5; up to 384^3 phases
-// (33 steps 10.2 / 9.3).  Over 64^3 to 1024^3, three orders and 33 to 250 steps
-// the choice is at most 5 % behind the better of the two.
+// A step of a chunk (16 planes) waits for the one before in the queue and takes
+// 9.8 / 10.4 / 12.4 us (7 / 13 / 25 points) for every 140 tiles, full rounds or 1.28
+// times their part, whichever is more.  A chunk can step as far as its successors
+// are in, so of the S chunks' n steps a triangle runs beside the uploads, and one
+// beside the downloads; the first hides less of its time, the reads of the host
+// arrays being the slower side.  Fitted to 372 calls of 33 to 250 steps over 23
+// grids (10 MB to 4.3 GB an array, planes of 32 to 2000 tiles, 30 to 2048 of them):
+// 5 % rms beyond 100 MB.  Pinned arrays, ms in chunks / in phases: 7 points 1024^3
+// 33 steps 122 / 173, 64 steps 215 / 227, 100 steps 324 / 294; 512^3 33 steps 19.5 /
+// 21.3, 48 steps 25.7 / 24.6; 25 points 1024^3 33 steps 140 / 185, 100 steps 379 / 335;
+// 64 x 1024 x 1024 33 steps 14.1 / 12.3, 576 x 300 x 900 33.6 / 28.5.
 bool chunks_faster(const st3d_ctx* c, uint32_t iterations) {
-  const double bytes = (double)host_array_bytes(c);
+  const double bytes = (double)host_array_bytes(c), n = (double)iterations;
   const double up = 3.0 * bytes / 211e3, down = 2.0 * bytes / 194e3;  // the link's rates
-  const double item = c->R == 1 ? 11.0 : c->R == 2 ? 11.6 : 14.3;
-  const double chunks = (double)((c->grid.xs + 15) / 16), tiles = (double)c->tma->ntj * c->tma->ntk;
-  return 0.2 * up + iterations * chunks * item * std::max(1.0, tiles / 108.0) <
-         up + down + steps_us(c, iterations);
+  const double S = (double)((c->grid.xs + 15) / 16), rounds = c->tma->ntj * (double)c->tma->ntk / 140.0;
+  const double step = (c->R == 1 ? 9.8 : c->R == 2 ? 10.4 : 12.4) * std::max(std::ceil(rounds), 1.28 * rounds);
+  const double work = n * S * step;
+  const double triangle = (n >= S ? 0.5 * S * S : n * S - 0.5 * n * n) * step;
+  const double beside = std::min(up, 0.23 * triangle) + std::min(down, 1.5 * triangle);
+  return up + down + work - 1.1 * std::min(beside, work) < up + down + steps_us(c, iterations);
 }
 
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and

@@ -15,8 +15,8 @@ AUTO, DIRECT = S.api.HOST_AUTO, S.api.HOST_DIRECT
 
 
 @pytest.mark.parametrize("grid,points,steps,asked,taken", [
-    ((80, 1024, 1024, 4, 4, 4), 25, 33, AUTO, STREAMED),
-    ((80, 1024, 1024, 4, 4, 4), 7, 40, AUTO, STREAMED),
+    ((512, 512, 512, 4, 4, 4), 7, 33, AUTO, STREAMED),
+    ((64, 1024, 1024, 4, 4, 4), 25, 33, AUTO, DIRECT),  # too few chunks to hide the transfers
     ((64, 64, 64, 4, 4, 4), 7, 100, AUTO, DIRECT),
     ((64, 64, 64, 4, 4, 4), 7, 41, STREAMED, STREAMED),
     ((130, 150, 200, 4, 4, 4), 13, 33, STREAMED, STREAMED),
