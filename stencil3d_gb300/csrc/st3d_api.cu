@@ -1104,14 +1104,14 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
   static_cast<WaveLayout&>(*w) = taken;
   // beyond R + 1 planes, or the slowest of two neighbours could wait for the
   // other (16 / 20 / 26 / 32 planes, Gpts/s: 25 points, 1024^2 planes 439 / 467 /
-  // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497).  Above 240 MB coupling gains
-  // at 7 and 13 points (20 steps, free -> coupled, us: 7 points 272^3 865 -> 839, 288^3
-  // 1046 -> 986, 320^3 1494 -> 1225, 400 x 180 x 300 910 -> 788) and costs 25 points 1 %
-  // at most up to 300 MB.  Below 120 MB, where L2 holds the fields, it costs up to 5 %
-  // (200^3 363 -> 379).  Between the two it goes either way: 240^3 526 -> 479, 256^3
-  // 665 -> 620, 128 x 384 x 384 858 -> 775, but 600 x 160 x 200 764 -> 798, 500 x 128 x
-  // 256 624 -> 676, 420 x 140 x 260 692 -> 751 (long calls gain more, 60 steps 256^3 13 %);
-  // no size alone tells them apart, so these run free.
+  // 463 / 453, 13 points 512^3 506 / 542 / 539 / 497).  Coupled runs take the same
+  // time on every GPU, free ones differ between GPUs and shapes (7 points, 20 steps, us
+  // over five GPUs, free / coupled: 200^3 361-363 / 379, 240^3 488-526 / 473-480, 256^3
+  // 609-666 / 614-622, 272^3 806-865 / 839, 288^3 968-1046 / 983-993, 320^3 1400-1494 /
+  // 1184-1225; 500 x 128 x 256 624 / 676, 420 x 140 x 260 692 / 751, 300 x 250 x 190 620 /
+  // 593; 60 steps gain more: 256^3 1931-2084 / 1778-1797).  Free up to 240 MB, where
+  // coupling costs more than it gives on one of the GPUs or shapes; 25 points
+  // differ by 2 % at most.
   w->couple = bytes > 2.4e8 ? kWaveCouple : 1 << 28;
   w->limit_ns = 4000000000ull + (uint64_t)(bytes / 12.0 * n / 2.5);
   return true;
