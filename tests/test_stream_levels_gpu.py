@@ -69,3 +69,18 @@ def test_levels_are_four_to_thirty_two(steps, levels):
     v, s, u = wave_inputs(grid, 3)
     _, _, info = _run(grid, 7, steps, None, 0, (v, s, u), host_path=STREAMED)
     assert info.host_path == STREAMED and info.stream_levels == levels
+
+
+@pytest.mark.parametrize("grid,points,steps,levels", [
+    ((1000, 128, 128, 4, 4, 4), 25, 8, 0), ((1000, 128, 128, 4, 4, 4), 25, 16, 16),
+    ((300, 100, 100, 4, 4, 4), 7, 5, 0), ((160, 160, 160, 4, 4, 4), 13, 6, 0),
+    ((160, 160, 160, 4, 4, 4), 13, 7, 7), ((40, 300, 300, 4, 4, 4), 7, 4, 4)])
+def test_few_steps_of_long_grids_run_over_chunks(grid, points, steps, levels):
+    """Few steps, planes small beside the length: the chunks of planes are the
+    faster form (a row of tiles spans all planes)."""
+    v, s, u = wave_inputs(grid, 3)
+    v1, u1, info = _run(grid, points, steps, None, 0, (v, s, u))
+    assert info.host_path == STREAMED and info.stream_levels == levels
+    v2, u2, _ = _run(grid, points, steps, None, 0, (v, s, u), host_path=DIRECT, tile_j=16, stages=4)
+    np.testing.assert_array_equal(v1, v2)
+    np.testing.assert_array_equal(u1, u2)
