@@ -550,7 +550,12 @@ int enqueue_persistent(st3d_batch* b, uint32_t steps, const int2* items, int tot
 // the queue takes its units' planes (with their warm-up) at 0.6 us over the
 // CTAs, 3 us for the launch and a quarter of the longest unit for the tail
 // (24 grids 567 us a step, their 7 slowest alone 238).  Grids are taken in the
-// order of what their own launches save.
+// order of what their own launches save.  A queue that is left with some of the
+// grids loses more than that (its units balance worse, its launches fill less): 16
+// grids of 64 to 200 points, 12 steps, 3 alone 2684 us against 2410 as one queue, 10
+// of 100 to 300, 5 steps, 4 alone 1588 against 1399; 24 of 64 to 320, 12 steps, 14
+// alone 5703 against 5399.  So a mixed schedule has to promise 13 % (64 grids,
+// 20 steps, 33 alone: 22981 against 24571).
 std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
   const size_t n = b->ctx.size();
   std::vector<double> own(n, 1e300), share(n), unit(n);
@@ -589,7 +594,7 @@ std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
     return own[x] / share[x] < own[y] / share[y];
   });
   std::vector<char> alone(n, 0), best(n, 0);
-  double best_us = 1e300, mine = 0.0;
+  double best_us = 1e300, mine = 0.0, queue_us = 0.0;
   for (size_t k = 0; k <= order.size(); ++k) {
     if (k > 0) {
       alone[order[k - 1]] = 1;
@@ -602,11 +607,14 @@ std::vector<char> split_grids(const st3d_batch* b, uint32_t steps) {
         longest = std::max(longest, unit[gi]);
       }
     const double us = mine + (sum > 0.0 ? steps * (std::max(sum + 0.25 * longest, 0.75 * longest) + 3.0) : 0.0);
+    if (k == 0) queue_us = us;
     if (us < best_us) {
       best_us = us;
       best = alone;
     }
   }
+  const bool mixed = std::find(best.begin(), best.end(), 0) != best.end();
+  if (mixed && best_us > 0.87 * queue_us) std::fill(best.begin(), best.end(), 0);
   return best;
 }
 

@@ -2,6 +2,8 @@
 Bar: info.launches counts the kernel launches captured -- a step of the queue is
 one, a grid that steps by itself one for many steps -- and calls shorter than
 one before, longer, and shorter again end where the sequential schedule does."""
+import random
+
 import numpy as np
 import pytest
 
@@ -44,3 +46,13 @@ def test_a_longer_call_after_a_short_one():
     for (ua, va), (ub, vb) in zip(got, want):
         np.testing.assert_array_equal(ua, ub)
         np.testing.assert_array_equal(va, vb)
+
+
+def test_a_short_call_stays_in_the_queue():
+    """16 grids of 64 to 200 points: a few of them alone beside the queue were
+    slower at 12 steps (2684 against 2410 us), all alone faster at 60."""
+    rng = random.Random(2)
+    specs = [(tuple(rng.randint(64, 200) for _ in range(3)) + (4, 4, 4), 0, None) for _ in range(16)]
+    specs = [(g, rng.choice([7, 13, 25]), s) for g, _, s in specs]
+    assert _launches(specs, 12, "graph") == 12
+    assert _launches(specs, 60, "graph") < 60
