@@ -66,7 +66,9 @@ struct RadiusOf {
   static constexpr int value = (P == 25) ? 4 : (P == 13) ? 2 : 1;
 };
 
-template <int P, int MODE, int TJ, int NV>
+// MANY: mode R with rsteps > 1 (a launch of one step has no loop: 7 points 70 x
+// 187 x 423 12.4 us a step, 14.4 through it).
+template <int P, int MODE, int TJ, int NV, bool MANY>
 __global__ void __launch_bounds__((TJ + 1) * 32, 1)
     k_tma(const __grid_constant__ CUtensorMap umap, const __grid_constant__ CUtensorMap vmap,
           const __grid_constant__ CUtensorMap smap, Geom g, Coefs<float> cf,
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__((TJ + 1) * 32, 1)
           if (MODE == ST3D_MODE_REF) {
             // rsteps steps at once: u and s stay, so does the sum; v alone moves
             x = vv;
-            for (int m = 0; m < rsteps; ++m) {
+            for (int m = 0; m < (MANY ? rsteps : 1); ++m) {
               const P4 t = fma4(splat(-cf.K), cu, x);
               x = {__ffma2_rn(ss.a, acc.a, t.a), __ffma2_rn(ss.b, acc.b, t.b)};
             }
@@ -270,7 +272,10 @@ template <int P, int MODE, int TJ, int NV>
 cudaError_t launch_cfg(const TmaPlan& plan, const Geom& g, const Coefs<float>& cf, float* v,
                        int ubuf, int vbuf, int sbuf, const Source& src, int rsteps,
                        uint32_t* dev_status, cudaStream_t stream) {
-  auto kern = k_tma<P, MODE, TJ, NV>;
+  auto kern = k_tma<P, MODE, TJ, NV, false>;
+  if constexpr (MODE == ST3D_MODE_REF) {
+    if (rsteps > 1) kern = k_tma<P, MODE, TJ, NV, true>;
+  }
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
   if (e != cudaSuccess) return e;
@@ -309,11 +314,11 @@ int occupancy_mode(int tj, int nv, size_t smem) {
       return 0;
     return b;
   };
-  if (tj == 16 && nv == 3) n = probe(k_tma<P, MODE, 16, 3>, 17 * 32);
-  if (tj == 8 && nv == 3) n = probe(k_tma<P, MODE, 8, 3>, 9 * 32);
-  if (tj == 8 && nv == 4) n = probe(k_tma<P, MODE, 8, 4>, 9 * 32);
-  if (tj == 16 && nv == 2) n = probe(k_tma<P, MODE, 16, 2>, 17 * 32);
-  if (tj == 16 && nv == 4) n = probe(k_tma<P, MODE, 16, 4>, 17 * 32);
+  if (tj == 16 && nv == 3) n = probe(k_tma<P, MODE, 16, 3, MODE == ST3D_MODE_REF>, 17 * 32);
+  if (tj == 8 && nv == 3) n = probe(k_tma<P, MODE, 8, 3, MODE == ST3D_MODE_REF>, 9 * 32);
+  if (tj == 8 && nv == 4) n = probe(k_tma<P, MODE, 8, 4, MODE == ST3D_MODE_REF>, 9 * 32);
+  if (tj == 16 && nv == 2) n = probe(k_tma<P, MODE, 16, 2, MODE == ST3D_MODE_REF>, 17 * 32);
+  if (tj == 16 && nv == 4) n = probe(k_tma<P, MODE, 16, 4, MODE == ST3D_MODE_REF>, 17 * 32);
   cudaGetLastError();
   return n;
 }
