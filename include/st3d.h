@@ -124,8 +124,9 @@ typedef struct st3d_grid_desc {
  * row pad.  STREAMED (st3d_iterate_host only): the DIRECT path with the
  * transfers and the steps overlapped in one launch -- CTAs copying u, v and s
  * in while the others step what is already in (mode W, 4 to 32 steps: rows of
- * tiles, a pipeline of as many levels as steps; otherwise a wavefront over
- * chunks of `ichunk` planes along i, 16 when 0), and copying the result out
+ * tiles, a pipeline of as many levels as steps; otherwise, and for few steps of
+ * grids that are long along i, a wavefront over chunks of `ichunk` planes along
+ * i, 16 when 0), and copying the result out
  * as it is done; the same bits as the phase-by-phase call.  AUTO takes it for
  * FP32 contexts on the TMA kernel's default tiles without temporal blocking
  * when v, s and u are pinned, except for mode W calls of more than 32 steps
