@@ -1121,35 +1121,45 @@ bool plan_wave(const st3d_ctx* c, uint32_t steps, WavePlan* w, double* est_us, b
 
 namespace {
 
-// The streamed drop-in call of the wave form as one launch of the multi-step
-// kernel with its transfer CTAs: device views of the pinned host arrays.  It takes
-// as many levels as steps, so that columns reach their last step in the order they
-// came in (25 points 512^3, 20 steps in 20 / 10 / 7
-// levels: 12.9 / 15.6 / 17.9 ms; chunks of planes, st3d_stream.cu, 15.9).
-// *done = false where another way is the only one.
-int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32_t iterations, bool* done) {
-  const int n = (int)std::min<uint32_t>(iterations, 1u << 20), R = c->R, xs = (int)c->L.xs;
-  const st3d_grid_desc& gd = c->grid;
-  WavePlan w = *c->wave;
-  if (n < 4 || n > std::min(w.max_steps, kWaveLevels) || w.ctas < 64) return ST3D_OK;
-  WaveXfer x;
-  // 25 points 512^3, 20 steps, with 12 / 16 / 20 / 24 upload and 12 download
-  // CTAs: 13.8 / 12.9 / 12.3 / 12.6 ms a call
-  x.n_up = 20;
-  x.n_down = 12;
-  x.planes = 16;
-  const int ctas = w.ctas - x.n_up - x.n_down;
+// Transfer CTAs of the streamed call on the multi-step kernel (25 points 512^3, 20
+// steps, with 12 / 16 / 20 / 24 upload and 12 download CTAs: 13.8 / 12.9 / 12.3 /
+// 12.6 ms a call).
+constexpr int kRowsUp = 20, kRowsDown = 12;
+
+// Its layout for a call of n steps: as many levels as steps, so that columns reach
+// their last step in the order they came in (25 points 512^3, 20 steps in 20 / 10 / 7
+// levels: 12.9 / 15.6 / 17.9 ms; chunks of planes, st3d_stream.cu, 15.9).  False
+// where it does not take the call.
+bool rows_layout(const st3d_ctx* c, uint32_t steps, WavePlan* w) {
+  if (!c->wave || steps < 4 || steps > (uint32_t)std::min(c->wave->max_steps, kWaveLevels) || c->wave->ctas < 64)
+    return false;
+  const int n = (int)steps, R = c->R, ctas = c->wave->ctas - kRowsUp - kRowsDown;
+  *w = *c->wave;
   double best = 1e300;
   for (int nar = 0; nar < 2; ++nar) {
     WaveLayout v;
-    if (!wave_layout(w, nar, n, ctas, c->L, R, &v)) continue;
-    const double us = wave_turns(v, n) * (xs + 2 * R) * (nar ? 1.05 : 1.0);
+    if (!wave_layout(*c->wave, nar, n, ctas, c->L, R, &v)) continue;
+    const double us = wave_turns(v, n) * ((double)c->L.xs + 2 * R) * (nar ? 1.05 : 1.0);
     if (us < best) {
       best = us;
-      static_cast<WaveLayout&>(w) = v;
+      static_cast<WaveLayout&>(*w) = v;
     }
   }
-  if (best > 1e299) return ST3D_OK;
+  return best < 1e299;
+}
+
+// The streamed drop-in call of the wave form as one launch of the multi-step
+// kernel with its transfer CTAs: device views of the pinned host arrays.
+// *done = false where another way is the only one.
+int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32_t iterations, bool* done) {
+  const int n = (int)iterations;
+  const st3d_grid_desc& gd = c->grid;
+  WavePlan w = *c->wave;
+  if (!rows_layout(c, iterations, &w)) return ST3D_OK;
+  WaveXfer x;
+  x.n_up = kRowsUp;
+  x.n_down = kRowsDown;
+  x.planes = 16;
   w.couple = kWaveCouple;
   x.R = ref_geom(gd);
   x.s = static_cast<float*>(c->fld[2]);
@@ -1198,23 +1208,38 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
   return ST3D_OK;
 }
 
-// Whether a streamed wave call of so few steps runs faster over chunks of planes
-// (st3d_stream.cu) than over rows of tiles (iterate_host_wave).  Rows come in one
-// after the other, each over all planes: a grid that is long along i beside its
-// planes has few of them to overlap, and short pieces of each plane to move; the
-// more steps, the more the pipeline of levels gains on that.  Measured over 28
-// grids, three orders and 4 to 32 steps, ms in chunks / in rows: 25 points 1000 x
-// 128 x 128 8 steps 2.13 / 3.41, 16 steps 4.65 / 3.65; 1500 x 200 x 200 4 steps 5.48 /
-// 8.76, 8 steps 6.32 / 7.68, 16 steps 15.8 / 8.4; 256^3 4 steps 1.70 / 2.02, 8 steps
-// 1.88 / 1.98, 16 steps 3.17 / 1.98; 64 x 1024 x 1024 4 steps 7.76 / 5.30.  The choice is
-// at most 9 % behind up to 25 steps (25 points, 32 steps on thin planes 23 %).  Where
-// rows are not whole 16-byte words the rows of tiles were faster but for 800 x 300 x
-// 150 at 4 steps (6.7 / 7.1).
-bool few_steps_in_chunks(const st3d_grid_desc& g, int R, uint32_t n) {
-  const double plane = (double)g.ys * g.zs, length = g.xs / std::sqrt(plane);
-  if (length < 0.85) return false;
-  if (length < 1.5) return n <= 6;
-  return n <= (R == 4 ? 8u : 10u) + (g.xs * plane < 2e7 ? 4u : 0u);
+// Whether a streamed wave call of up to 16 steps runs faster over chunks of planes
+// (st3d_stream.cu) than over rows of tiles (iterate_host_wave); more steps gain from
+// the pipeline of levels.  Both forms are bound by their transfers here.  Rows of
+// tiles come in one after the other over all planes, so the slower direction is
+// overlapped but for some 5 rows, and a row's piece of a plane costs a download CTA
+// 1.7 us for every 39 KB of it (19 KB where rows are not whole 16-byte words).  Chunks
+// leave 15 % and some 6 chunks of the faster direction beside nothing, move rows that
+// are not whole words 2.4 times slower, and a step of a chunk takes 5.8 / 6.3 / 7.8 us
+// (7 / 13 / 25 points; less below 30 tiles, 2.8 of it a round of 140 above), which
+// adds to the transfers less than in full.  Fitted to 560 calls of each on 28 grids
+// (8 and 7 % rms; on 34 others the choice is 1 % behind the better on average, 19 %
+// at most), ms in chunks / in rows: 25 points 1000 x 128 x 128 8 steps 2.13 / 3.41, 16
+// steps 4.65 / 3.65; 1500 x 200 x 200 4 steps 5.48 / 8.76; 256^3 4 steps 1.70 / 2.02, 16
+// steps 3.17 / 1.98; 64 x 1024 x 1024 4 steps 7.76 / 5.30; 711 x 887 x 128 at 13 points
+// 14 steps 8.0 / 10.1; 279 x 367 x 25 4 steps 0.90 / 1.94.
+bool few_steps_in_chunks(const st3d_ctx* c, uint32_t n, bool whole) {
+  WavePlan w;
+  if (n > 16 || !rows_layout(c, n, &w)) return false;
+  const st3d_grid_desc& g = c->grid;
+  const double bytes = (double)host_array_bytes(c);
+  const double up = 3.0 * bytes / 211e3, down = 2.0 * bytes / 194e3;  // the link's rates
+  const WaveShape& sh = w.shape[w.narrow];
+  const double piece = sh.tj * (g.zs + 2.0 * g.zh) * 4.0;
+  const double out = std::max(down, 2.0 * sh.ntj * g.xs * std::ceil(piece / (whole ? 38912.0 : 19456.0)) * 1.7 / kRowsDown);
+  const double rows = 1.21 * std::max(up, out) + 4.73 / sh.ntj * std::min(up, out) + (6.0 + c->R) * (n - 1);
+  const double S = (double)((g.xs + 15) / 16), tiles = (double)c->tma->ntj * c->tma->ntk, slow = whole ? 1.0 : 2.43;
+  const double step = (c->R == 1 ? 5.77 : c->R == 2 ? 6.25 : 7.83) *
+                      std::max(tiles > 140.0 ? std::ceil(tiles / 140.0) : std::min(1.0, std::pow(tiles / 30.0, 0.6)),
+                               2.77 * tiles / 140.0);
+  const double move = slow * (up + down * std::min(1.0, 0.155 + 5.7 / S)), work = n * S * step;
+  const double chunks = std::pow(std::pow(move, 1.65) + std::pow(work, 1.65), 1.0 / 1.65) + 116.0;
+  return chunks < rows;
 }
 
 // Time of n wave steps of a call as the launches st3d_iterate makes of them, us.
@@ -1248,16 +1273,18 @@ double steps_us(const st3d_ctx* c, uint32_t n) {
 // 5 % rms beyond 100 MB.  Pinned arrays, ms in chunks / in phases: 7 points 1024^3
 // 33 steps 122 / 173, 64 steps 215 / 227, 100 steps 324 / 294; 512^3 33 steps 19.5 /
 // 21.3, 48 steps 25.7 / 24.6; 25 points 1024^3 33 steps 140 / 185, 100 steps 379 / 335;
-// 64 x 1024 x 1024 33 steps 14.1 / 12.3, 576 x 300 x 900 33.6 / 28.5.
-bool chunks_faster(const st3d_ctx* c, uint32_t iterations) {
+// 64 x 1024 x 1024 33 steps 14.1 / 12.3, 576 x 300 x 900 33.6 / 28.5; rows that are not
+// whole 16-byte words (7 points 329 x 276 x 1203) 34.4 / 18.0.
+bool chunks_faster(const st3d_ctx* c, uint32_t iterations, bool whole) {
   const double bytes = (double)host_array_bytes(c), n = (double)iterations;
   const double up = 3.0 * bytes / 211e3, down = 2.0 * bytes / 194e3;  // the link's rates
   const double S = (double)((c->grid.xs + 15) / 16), rounds = c->tma->ntj * (double)c->tma->ntk / 140.0;
   const double step = (c->R == 1 ? 9.8 : c->R == 2 ? 10.4 : 12.4) * std::max(std::ceil(rounds), 1.28 * rounds);
   const double work = n * S * step;
   const double triangle = (n >= S ? 0.5 * S * S : n * S - 0.5 * n * n) * step;
-  const double beside = std::min(up, 0.23 * triangle) + std::min(down, 1.5 * triangle);
-  return up + down + work - 1.1 * std::min(beside, work) < up + down + steps_us(c, iterations);
+  const double slow = whole ? 1.0 : 2.43;  // rows that are not whole 16-byte words
+  const double beside = std::min(slow * up, 0.23 * triangle) + std::min(slow * down, 1.5 * triangle);
+  return slow * (up + down) + work - 1.1 * std::min(beside, work) < up + down + steps_us(c, iterations);
 }
 
 // The streamed drop-in call (st3d_stream.cu): upload, `iterations` steps and
@@ -1278,12 +1305,12 @@ int iterate_host_streamed(st3d_ctx* c, void* v, const void* s, void* u, uint32_t
   const float* hs = static_cast<const float*>(direct_view(s, hbytes));
   const float* hu = static_cast<const float*>(direct_view(u, hbytes));
   if (!hv || !hs || !hu) return ST3D_OK;
-  if (hp == ST3D_HOST_AUTO && c->opts.mode == ST3D_MODE_WAVE && iterations > (uint32_t)kWaveLevels &&
-      (c->wave || c->brick.nbi > 0) && !chunks_faster(c, iterations))
-    return ST3D_OK;
   const bool whole = (reinterpret_cast<uintptr_t>(hu) | reinterpret_cast<uintptr_t>(hv) |
                       reinterpret_cast<uintptr_t>(hs)) % 16 == 0 && c->grid.zh % 4 == 0 && c->grid.zs % 4 == 0;
-  if (c->wave && !(whole && few_steps_in_chunks(c->grid, c->R, iterations))) {
+  if (hp == ST3D_HOST_AUTO && c->opts.mode == ST3D_MODE_WAVE && iterations > (uint32_t)kWaveLevels &&
+      (c->wave || c->brick.nbi > 0) && !chunks_faster(c, iterations, whole))
+    return ST3D_OK;
+  if (c->wave && !few_steps_in_chunks(c, iterations, whole)) {
     const int rc = iterate_host_wave(c, const_cast<float*>(hv), hs, const_cast<float*>(hu), iterations, done);
     if (rc != ST3D_OK || *done) return rc;
   }
