@@ -73,7 +73,7 @@ def test_levels_are_four_to_thirty_two(steps, levels):
 
 @pytest.mark.parametrize("grid,points,steps,levels", [
     ((1000, 128, 128, 4, 4, 4), 25, 8, 0), ((1000, 128, 128, 4, 4, 4), 25, 16, 16),
-    ((300, 100, 100, 4, 4, 4), 7, 5, 0), ((160, 160, 160, 4, 4, 4), 13, 6, 0),
+    ((300, 100, 100, 4, 4, 4), 7, 5, 0), ((279, 367, 25, 4, 4, 4), 25, 4, 0), ((160, 160, 160, 4, 4, 4), 13, 6, 0),
     ((160, 160, 160, 4, 4, 4), 13, 7, 7), ((40, 300, 300, 4, 4, 4), 7, 4, 4)])
 def test_few_steps_of_long_grids_run_over_chunks(grid, points, steps, levels):
     """Few steps, planes small beside the length: the chunks of planes are the

@@ -18,6 +18,7 @@ AUTO, DIRECT = S.api.HOST_AUTO, S.api.HOST_DIRECT
     ((512, 512, 512, 4, 4, 4), 7, 33, AUTO, STREAMED),
     ((64, 1024, 1024, 4, 4, 4), 25, 33, AUTO, DIRECT),  # too few chunks to hide the transfers
     ((64, 64, 64, 4, 4, 4), 7, 100, AUTO, DIRECT),
+    ((120, 276, 603, 4, 4, 4), 7, 33, AUTO, DIRECT),  # rows that are not whole 16-byte words
     ((64, 64, 64, 4, 4, 4), 7, 41, STREAMED, STREAMED),
     ((130, 150, 200, 4, 4, 4), 13, 33, STREAMED, STREAMED),
     ((130, 150, 200, 4, 4, 4), 13, 120, AUTO, DIRECT),
