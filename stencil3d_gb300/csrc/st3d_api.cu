@@ -1218,8 +1218,8 @@ int iterate_host_wave(st3d_ctx* c, float* hv, const float* hs, float* hu, uint32
 // are not whole words 2.4 times slower, and a step of a chunk takes 5.8 / 6.3 / 7.8 us
 // (7 / 13 / 25 points; less below 30 tiles, 2.8 of it a round of 140 above), which
 // adds to the transfers less than in full.  Fitted to 560 calls of each on 28 grids
-// (8 and 7 % rms; on 34 others the choice is 1 % behind the better on average, 19 %
-// at most), ms in chunks / in rows: 25 points 1000 x 128 x 128 8 steps 2.13 / 3.41, 16
+// (8 and 7 % rms; on 34 others the choice is 1 % behind the better on average, 17 %
+// at most; more than 10 steps have to promise 8 %), ms in chunks / in rows: 25 points 1000 x 128 x 128 8 steps 2.13 / 3.41, 16
 // steps 4.65 / 3.65; 1500 x 200 x 200 4 steps 5.48 / 8.76; 256^3 4 steps 1.70 / 2.02, 16
 // steps 3.17 / 1.98; 64 x 1024 x 1024 4 steps 7.76 / 5.30; 711 x 887 x 128 at 13 points
 // 14 steps 8.0 / 10.1; 279 x 367 x 25 4 steps 0.90 / 1.94.
@@ -1239,7 +1239,7 @@ bool few_steps_in_chunks(const st3d_ctx* c, uint32_t n, bool whole) {
                                2.77 * tiles / 140.0);
   const double move = slow * (up + down * std::min(1.0, 0.155 + 5.7 / S)), work = n * S * step;
   const double chunks = std::pow(std::pow(move, 1.65) + std::pow(work, 1.65), 1.0 / 1.65) + 116.0;
-  return chunks < rows;
+  return (n > 10 ? 1.08 : 1.0) * chunks < rows;
 }
 
 // Time of n wave steps of a call as the launches st3d_iterate makes of them, us.
@@ -1265,21 +1265,23 @@ double steps_us(const st3d_ctx* c, uint32_t n) {
 // (st3d_stream.cu) or phase by phase, the steps many a launch with all CTAs.
 // A step of a chunk (16 planes) waits for the one before in the queue and takes
 // 9.8 / 10.4 / 12.4 us (7 / 13 / 25 points) for every 140 tiles, full rounds or 1.28
-// times their part, whichever is more.  A chunk can step as far as its successors
-// are in, so of the S chunks' n steps a triangle runs beside the uploads, and one
-// beside the downloads; the first hides less of its time, the reads of the host
-// arrays being the slower side.  Fitted to 372 calls of 33 to 250 steps over 23
-// grids (10 MB to 4.3 GB an array, planes of 32 to 2000 tiles, 30 to 2048 of them):
-// 5 % rms beyond 100 MB.  Pinned arrays, ms in chunks / in phases: 7 points 1024^3
-// 33 steps 122 / 173, 64 steps 215 / 227, 100 steps 324 / 294; 512^3 33 steps 19.5 /
-// 21.3, 48 steps 25.7 / 24.6; 25 points 1024^3 33 steps 140 / 185, 100 steps 379 / 335;
-// 64 x 1024 x 1024 33 steps 14.1 / 12.3, 576 x 300 x 900 33.6 / 28.5; rows that are not
-// whole 16-byte words (7 points 329 x 276 x 1203) 34.4 / 18.0.
+// times their part (1.4 of a single one), whichever is more.  A chunk can step as
+// far as its successors are in, so of the S chunks' n steps a triangle runs beside
+// the uploads, and one beside the downloads; the first hides less of its time, the
+// reads of the host arrays being the slower side.  Fitted to 372 calls of 33 to 250
+// steps over 23 grids (10 MB to 4.3 GB an array, planes of 32 to 2000 tiles, 30 to
+// 2048 of them): 5 % rms beyond 100 MB, the choice at most 4 % behind the better.
+// Pinned arrays, ms in chunks / in phases: 7 points 1024^3 33 steps 122 / 173, 64 steps
+// 215 / 227, 100 steps 324 / 294; 512^3 33 steps 19.5 / 21.3, 48 steps 25.7 / 24.6; 25
+// points 1024^3 33 steps 140 / 185, 100 steps 379 / 335; 64 x 1024 x 1024 33 steps 14.1 /
+// 12.3, 576 x 300 x 900 33.6 / 28.5; rows that are not whole 16-byte words (7 points 329
+// x 276 x 1203) 34.4 / 18.0.
 bool chunks_faster(const st3d_ctx* c, uint32_t iterations, bool whole) {
   const double bytes = (double)host_array_bytes(c), n = (double)iterations;
   const double up = 3.0 * bytes / 211e3, down = 2.0 * bytes / 194e3;  // the link's rates
   const double S = (double)((c->grid.xs + 15) / 16), rounds = c->tma->ntj * (double)c->tma->ntk / 140.0;
-  const double step = (c->R == 1 ? 9.8 : c->R == 2 ? 10.4 : 12.4) * std::max(std::ceil(rounds), 1.28 * rounds);
+  const double step = (c->R == 1 ? 9.8 : c->R == 2 ? 10.4 : 12.4) *
+                      (rounds <= 1.0 ? std::max(1.0, 1.4 * rounds) : std::max(std::ceil(rounds), 1.28 * rounds));
   const double work = n * S * step;
   const double triangle = (n >= S ? 0.5 * S * S : n * S - 0.5 * n * n) * step;
   const double slow = whole ? 1.0 : 2.43;  // rows that are not whole 16-byte words
